@@ -51,10 +51,14 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[sizeof(NoAllocS
 
 // kernels shared with olv_bfs (bfs.cu)
 __global__ void k_fill_i32(int32_t *__restrict__ a, uint32_t n, int32_t x);
-__global__ void k_bfs_init(TravCtl *c, int32_t *level, uint32_t *q0, const uint32_t *rowptr,
-                           uint32_t src, unsigned long long E);
-__global__ void k_bfs_begin(TravCtl *c, uint32_t V, float alpha, float beta);
-__global__ void k_bfs_end(TravCtl *c, cudaGraphConditionalHandle h, int use_cond, uint32_t V);
+__global__ void k_bfs_init(TravCtl *c, int32_t *level, uint32_t *q0, uint32_t *q1,
+                           const uint32_t *rowptr, const uint32_t *col, uint32_t src, uint32_t V,
+                           unsigned long long E, int fill, float alpha, float beta,
+                           cudaGraphConditionalHandle h, int use_cond);
+__global__ void k_bfs_end(TravCtl *c, cudaGraphConditionalHandle h, int use_cond, uint32_t V,
+                          uint32_t *q0, uint32_t *q1, const uint32_t *rowptr, const uint32_t *col,
+                          float alpha, float beta);
+constexpr int kSmallThreads = 1024;   // their one CTA
 
 struct NoAllocBfsOp {
     using SV = uint32_t;
@@ -187,7 +191,9 @@ extern "C" int olv_bfs_noalloc(const uint32_t *rowptr, const uint32_t *col, uint
     }
 
     k_fill_i32<<<sms * 8, kBlock, 0, s>>>(level_out, V, kInf);
-    k_bfs_init<<<1, 1, 0, s>>>(ctl, level_out, sc->q0, rowptr, src, (unsigned long long)E);
+    const float never_pull = 0.0f, beta = 24.0f;
+    k_bfs_init<<<1, kSmallThreads, 0, s>>>(ctl, level_out, sc->q0, sc->q1, rowptr, col, src, V,
+                                           (unsigned long long)E, 0, never_pull, beta, 0, 0);
     AdvanceArgs a;
     a.rbeg = rowptr;
     a.rend = rowptr + 1;
@@ -205,14 +211,13 @@ extern "C" int olv_bfs_noalloc(const uint32_t *rowptr, const uint32_t *col, uint
     NoAllocBfsOp op = {};
     op.rowptr = rowptr;
     op.V = V;
-    const float never_pull = 0.0f, beta = 24.0f;
     int batch = 4;
     for (;;) {
         for (int i = 0; i < batch; i++) {
-            k_bfs_begin<<<1, 1, 0, s>>>(ctl, V, never_pull, beta);
             k_advance_chunks<NoAllocBfsOp><<<sms * 4, kBlock, 0, s>>>(a, op);
             k_advance_pieces<NoAllocBfsOp><<<sms * 4, kBlock, 0, s>>>(a, op);
-            k_bfs_end<<<1, 1, 0, s>>>(ctl, 0, 0, V);
+            k_bfs_end<<<1, kSmallThreads, 0, s>>>(ctl, 0, 0, V, sc->q0, sc->q1, rowptr, col,
+                                                  never_pull, beta);
         }
         OLV_CUDA(cudaGetLastError());
         unsigned int done = 0;
