@@ -171,8 +171,7 @@ __device__ __forceinline__ void warp_add64(unsigned long long x, unsigned long l
     if (lane_id() == 0 && x) atomicAdd(dst, x);
 }
 
-// Exclusive scan over the CTA (blockDim.x == T).  s_warp holds 33 words.
-template <int T = kBlock>
+// Exclusive scan over the CTA (blockDim.x == kBlock).  s_warp holds 33 words.
 __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t x, uint32_t *total,
                                                          uint32_t *s_warp) {
     const uint32_t lane = lane_id(), wid = threadIdx.x >> 5;
@@ -185,7 +184,7 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t x, uint32_t *t
     if (lane == 31) s_warp[wid] = incl;
     __syncthreads();
     if (wid == 0) {
-        constexpr int NW = T / 32;
+        constexpr int NW = kBlock / 32;
         uint32_t t = lane < NW ? s_warp[lane] : 0;
         uint32_t ti = t;
 #pragma unroll

@@ -28,6 +28,7 @@
 #include "olive_b200/olv_advance.cuh"
 #include "olv_graphexec.cuh"
 #include "olv_internal.cuh"
+#include "olv_small.cuh"
 
 namespace olv {
 
@@ -93,24 +94,16 @@ __global__ void k_fill_i32(int32_t *__restrict__ a, uint32_t n, int32_t x) {
 // about 15 us whatever its size (its launches are nearly empty there), while a
 // frontier of a few hundred vertices is a few dependent memory round trips of
 // work: about 2 us here.  So the kernel that ends a superstep also runs every following
-// level itself, one after another, as long as the frontier is at most
-// kSmallCap vertices (what two entries per thread cover) with at most
-// kSmallEdges out-edges (four rounds of kSmallItems edges per thread: about
-// the time of one superstep of the chain).  The frontier stays in shared
+// level itself, one after another, as long as the frontier is small
+// (olv_small.cuh).  The frontier stays in shared
 // memory with its row ranges, loaded beside the claim that found the vertex,
 // so a level's chain is: column -> claim and row range -> push.  Measured on
 // a 128 x 128 grid (about 200 levels): 3.94 -> 0.42 ms a call; the first and
 // last levels of a uniform digraph of 1,000,003 vertices: 380 -> 289 us, of
 // RMAT-24: 594 -> 554 us (there also two launches fewer per superstep).
-constexpr int kSmallThreads = 1024;
-constexpr uint32_t kSmallCap = 2 * kSmallThreads;
-constexpr uint32_t kSmallEdges = 16384;
-constexpr int kSmallItems = 4;
-
 struct SmallShared {
-    uint32_t beg[kSmallCap], off[kSmallCap];                  // the level being expanded
+    SmallIndex ix;                                            // the level being expanded
     uint32_t v[kSmallCap], obeg[kSmallCap], odeg[kSmallCap];  // the next one
-    uint32_t warp[33];
     uint32_t n;
     int go;
     unsigned long long m_last, m_all;
@@ -144,9 +137,58 @@ __device__ __forceinline__ bool bfs_small_ok(const TravCtl *c) {
     return !c->done && !c->queue_stale && c->qsize[c->cur] <= kSmallCap && c->m_f <= kSmallEdges;
 }
 
+// Edges base .. base + 1024 N - 1 of the level in sh (N per thread in flight):
+// claims, and pushes of the vertices claimed.  Returns the out-edges of those
+// this thread claimed.
+template <int N>
+__device__ __forceinline__ uint32_t bfs_small_edges(uint32_t base, uint32_t total, int next,
+                                                    int32_t *level, uint32_t *q,
+                                                    const uint32_t *__restrict__ rowptr,
+                                                    const uint32_t *__restrict__ col,
+                                                    SmallShared &sh) {
+    // each stage issues all its loads or atomics before any result is used
+    uint32_t at[N], v[N], rb[N], re[N], pos[N], found = 0;
+    int was[N];
+    bool act[N], won[N];
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        const uint32_t k = base + j * kSmallThreads + threadIdx.x;
+        act[j] = k < total;
+        at[j] = 0;
+        if (act[j]) {
+            const uint32_t lo = sh.ix.owner(k);
+            at[j] = sh.ix.beg[lo] + (k - sh.ix.off[lo]);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < N; j++) v[j] = act[j] ? __ldg(&col[at[j]]) : 0u;
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        was[j] = act[j] ? atomicCAS(&level[v[j]], kInf, next) : 0;
+        rb[j] = act[j] ? __ldg(&rowptr[v[j]]) : 0u;
+        re[j] = act[j] ? __ldg(&rowptr[v[j] + 1]) : 0u;
+    }
+#pragma unroll
+    for (int j = 0; j < N; j++) won[j] = act[j] && was[j] == kInf;
+    small_place(won, &sh.n, pos);
+#pragma unroll
+    for (int j = 0; j < N; j++)
+        if (won[j]) {
+            found += re[j] - rb[j];
+            if (pos[j] < kSmallCap) {
+                sh.v[pos[j]] = v[j];
+                sh.obeg[pos[j]] = rb[j];
+                sh.odeg[pos[j]] = re[j] - rb[j];
+            } else {
+                q[pos[j]] = v[j];
+            }
+        }
+    return found;
+}
+
 // Whole CTA: levels from the current queue until the frontier is empty or too
 // large; leaves the frontier in the same queue.
-__device__ void bfs_small(TravCtl *c, uint32_t V, uint32_t *q0, uint32_t *q1,
+__device__ void bfs_small(TravCtl *c, uint32_t *q0, uint32_t *q1,
                           const uint32_t *__restrict__ rowptr, const uint32_t *__restrict__ col,
                           SmallShared &sh) {
     int32_t *level = static_cast<int32_t *>(c->vdata);
@@ -154,7 +196,7 @@ __device__ void bfs_small(TravCtl *c, uint32_t V, uint32_t *q0, uint32_t *q1,
     uint32_t n = c->qsize[c->cur];
     const uint32_t lv0 = c->level;
     uint32_t lv = lv0;
-    const uint32_t t = threadIdx.x, lane = lane_id();
+    const uint32_t t = threadIdx.x;
     for (uint32_t i = t; i < n; i += kSmallThreads) {
         const uint32_t v = q[i], b = __ldg(&rowptr[v]);
         sh.v[i] = v;
@@ -170,75 +212,20 @@ __device__ void bfs_small(TravCtl *c, uint32_t V, uint32_t *q0, uint32_t *q1,
     uint32_t m_last = 0;                         // those of the last level
     __syncthreads();
     while (n > 0 && n <= kSmallCap) {
-        const uint32_t i0 = 2 * t;
-        const uint32_t d0 = i0 < n ? sh.odeg[i0] : 0, d1 = i0 + 1 < n ? sh.odeg[i0 + 1] : 0;
-        const uint32_t b0 = i0 < n ? sh.obeg[i0] : 0, b1 = i0 + 1 < n ? sh.obeg[i0 + 1] : 0;
-        uint32_t total;
-        const uint32_t off = block_exclusive_scan<kSmallThreads>(d0 + d1, &total, sh.warp);
+        const uint32_t total = sh.ix.number(
+            n, lv, [&](uint32_t i) { return sh.odeg[i]; }, [&](uint32_t i) { return sh.obeg[i]; });
         if (total > kSmallEdges) break;
-        sh.beg[i0] = b0;
-        sh.off[i0] = off;
-        sh.beg[i0 + 1] = b1;
-        sh.off[i0 + 1] = off + d0;
         if (t == 0) sh.n = 0;
         __syncthreads();
         m_last = 0;
         const int next = (int)lv + 1;
-        for (uint32_t base = 0; base < total; base += kSmallThreads * kSmallItems) {
-            uint32_t v[kSmallItems], rb[kSmallItems], re[kSmallItems];
-            int r[kSmallItems];
-            bool act[kSmallItems];
-#pragma unroll
-            for (int j = 0; j < kSmallItems; j++) {
-                const uint32_t k = base + j * kSmallThreads + t;
-                act[j] = k < total;
-                v[j] = 0;
-                if (act[j]) {
-                    uint32_t lo = 0;   // the last entry whose offset is <= k owns slot k
-#pragma unroll
-                    for (uint32_t step = kSmallCap / 2; step > 0; step >>= 1)
-                        if (sh.off[lo + step] <= k) lo += step;
-                    v[j] = __ldg(&col[sh.beg[lo] + (k - sh.off[lo])]);
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < kSmallItems; j++) {
-                r[j] = 0;
-                if (act[j]) {
-                    r[j] = atomicCAS(&level[v[j]], kInf, next);
-                    rb[j] = __ldg(&rowptr[v[j]]);
-                    re[j] = __ldg(&rowptr[v[j] + 1]);
-                }
-            }
-            unsigned m[kSmallItems];
-            uint32_t tot = 0;
-#pragma unroll
-            for (int j = 0; j < kSmallItems; j++) {
-                m[j] = __ballot_sync(0xffffffffu, r[j] == kInf);
-                tot += __popc(m[j]);
-            }
-            if (tot) {
-                uint32_t pos = 0;
-                if (lane == 0) pos = atomicAdd(&sh.n, tot);
-                pos = __shfl_sync(0xffffffffu, pos, 0);
-#pragma unroll
-                for (int j = 0; j < kSmallItems; j++) {
-                    if (r[j] == kInf) {
-                        const uint32_t p = pos + __popc(m[j] & ((1u << lane) - 1u));
-                        const uint32_t deg = re[j] - rb[j];
-                        m_last += deg;
-                        if (p < kSmallCap) {
-                            sh.v[p] = v[j];
-                            sh.obeg[p] = rb[j];
-                            sh.odeg[p] = deg;
-                        } else {
-                            q[p] = v[j];
-                        }
-                    }
-                    pos += __popc(m[j]);
-                }
-            }
-        }
+        if (total <= kSmallThreads)
+            m_last = bfs_small_edges<1>(0, total, next, level, q, rowptr, col, sh);
+        else if (total <= 2 * kSmallThreads)
+            m_last = bfs_small_edges<2>(0, total, next, level, q, rowptr, col, sh);
+        else
+            for (uint32_t base = 0; base < total; base += kSmallThreads * kSmallItems)
+                m_last += bfs_small_edges<kSmallItems>(base, total, next, level, q, rowptr, col, sh);
         m_all += m_last;
         reached += n;
         edges += total;
@@ -290,7 +277,7 @@ k_bfs_init(TravCtl *c, int32_t *level, uint32_t *q0, uint32_t *q1, const uint32_
         sh.go = bfs_small_ok(c);
     }
     __syncthreads();
-    if (sh.go) bfs_small(c, V, q0, q1, rowptr, col, sh);
+    if (sh.go) bfs_small(c, q0, q1, rowptr, col, sh);
     if (threadIdx.x == 0) {
         bfs_begin(c, V, alpha, beta);
         if (use_cond) cudaGraphSetConditional(h, c->done ? 0u : 1u);
@@ -633,7 +620,7 @@ k_bfs_end(TravCtl *c, cudaGraphConditionalHandle h, int use_cond, uint32_t V, ui
         sh.go = bfs_small_ok(c);
     }
     __syncthreads();
-    if (sh.go) bfs_small(c, V, q0, q1, rowptr, col, sh);
+    if (sh.go) bfs_small(c, q0, q1, rowptr, col, sh);
     if (threadIdx.x == 0) {
         bfs_begin(c, V, alpha, beta);
         if (use_cond) cudaGraphSetConditional(h, c->done ? 0u : 1u);
@@ -644,8 +631,11 @@ k_bfs_end(TravCtl *c, cudaGraphConditionalHandle h, int use_cond, uint32_t V, ui
 int traversal_workspace(olv_graph *g, bool pieces) {
     Workspace &w = g->ws;
     const size_t V = g->V;
-    OLV_TRY(w.q0.ensure(V * 4 + 16));
-    OLV_TRY(w.q1.ensure(V * 4 + 16));
+    // SSSP's small supersteps may queue a vertex more than once, at most once
+    // per edge
+    const size_t qn = V > kSmallEdges ? V : kSmallEdges;
+    OLV_TRY(w.q0.ensure(qn * 4 + 16));
+    OLV_TRY(w.q1.ensure(qn * 4 + 16));
     OLV_TRY(w.ctl.ensure(sizeof(TravCtl)));
     OLV_TRY(w.fbits.ensure(2 * (((size_t)V + 31) / 32 + 8) * 4));
     if (pieces) {

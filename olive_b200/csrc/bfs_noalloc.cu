@@ -30,6 +30,7 @@
 
 #include "olive_b200/olv_advance.cuh"
 #include "olv_internal.cuh"
+#include "olv_small.cuh"
 
 namespace olv {
 
@@ -58,7 +59,6 @@ __global__ void k_bfs_init(TravCtl *c, int32_t *level, uint32_t *q0, uint32_t *q
 __global__ void k_bfs_end(TravCtl *c, cudaGraphConditionalHandle h, int use_cond, uint32_t V,
                           uint32_t *q0, uint32_t *q1, const uint32_t *rowptr, const uint32_t *col,
                           float alpha, float beta);
-constexpr int kSmallThreads = 1024;   // their one CTA
 
 struct NoAllocBfsOp {
     using SV = uint32_t;

@@ -62,11 +62,11 @@
 #include "olive_b200/olv_advance.cuh"
 #include "olv_graphexec.cuh"
 #include "olv_internal.cuh"
+#include "olv_small.cuh"
 
 namespace olv {
 
 int traversal_workspace(olv_graph *g, bool pieces);
-__global__ void k_fill_i32(int32_t *__restrict__ a, uint32_t n, int32_t x);
 
 constexpr uint32_t kModeRelax = 0;
 constexpr uint32_t kModeSplit = 2;
@@ -261,34 +261,6 @@ struct SsspOp {
 };
 
 __device__ void sssp_begin(TravCtl *c);
-
-__global__ void k_sssp_init(TravCtl *c, uint32_t *dist, uint32_t *q0, uint32_t src,
-                            uint32_t delta, uint32_t sub, uint32_t sub_buckets,
-                            uint32_t tail_width, uint32_t route, uint32_t direct_min,
-                            const uint32_t *newid) {
-    if (newid) src = newid[src];   // relabelled run: the source's new id
-    TravCtl t = {};
-    t.qsize[0] = 1;
-    t.vdata = dist;
-    t.delta = delta;
-    t.bucket_end = delta;
-    t.sub_width = sub < delta ? sub : 0;
-    t.sub_buckets = sub_buckets;
-    t.heavy_index = 0;
-    t.tail_width = tail_width > delta ? tail_width : 0;
-    t.all_edges = 0;
-    t.route = t.tail_width != 0 && route;
-    t.direct_min = t.route ? direct_min : 0;
-    t.threshold = (t.sub_width && sub_buckets > 0) ? t.sub_width : delta;
-    t.epoch = 1;
-    t.far_min = 0xffffffffu;
-    t.heavy_done = 0;
-    t.bucket_lo = 0;
-    *c = t;
-    dist[src] = 0;
-    q0[0] = src;
-    sssp_begin(c);
-}
 
 static __device__ __forceinline__ uint32_t sat_add(uint32_t a, uint32_t b) {
     const uint64_t t = (uint64_t)a + b;
@@ -849,9 +821,427 @@ __device__ void sssp_end_step(TravCtl *c, cudaGraphConditionalHandle h, int use_
     if (use_cond) cudaGraphSetConditional(h, c->done ? 0u : 1u);
 }
 
-__global__ void k_sssp_end(TravCtl *c, cudaGraphConditionalHandle h, int use_cond,
-                           uint32_t max_steps, uint32_t bl_cap) {
-    sssp_end_step(c, h, use_cond, max_steps, bl_cap);
+// ------------------------------------------------------ small supersteps --
+// Relax and split supersteps whose input fits one CTA.  The kernel chain
+// costs about 17 us a superstep whatever its size (four launches), and a
+// graph of long diameter has hundreds of supersteps of a few hundred vertices
+// each.  So the kernel that ends a superstep runs the following ones itself
+// while they are relax steps of at most kSmallCap vertices (two per thread)
+// with at most kSmallEdges edges, or splits of at most kSmallFar pile entries;
+// the control block is copied to shared memory meanwhile and the same end
+// step moves from one superstep to the next.  The near queue stays in shared
+// memory with its row ranges, loaded beside the relaxation, so a superstep's
+// chain is: edge and source distance -> atomicMin and row range -> push.
+// Piles, their marks and the bucket list are kept as the kernel chain keeps
+// them, the near marks are empty here and set again for the queue that is
+// handed back, so a run can change over at any superstep.
+// What bounds it: dependent L2 round trips of one SM (about 4 us a superstep of
+// 1300 edges).  Measured: 301 x 517 grid, weights U[1,255], 815 supersteps
+// 13.9 -> 3.3 ms; RMAT-24 1.69 -> 1.66 ms (its last supersteps; also the
+// distances and marks cleared by one launch).
+constexpr uint32_t kSmallFar = 16384;
+constexpr uint32_t kSmallHash = 1024;
+
+struct SsspSmall {
+    const uint2 *lr;            // light ranges per vertex
+    const uint32_t *rowptr;     // full rows
+    const uint2 *cw;            // (column, weight) pairs, light | heavy
+    uint32_t *q0, *q1, *far0, *far1;
+    uint32_t *nmark0, *nmark1;
+    FarMarks fm;
+    uint32_t *blist;
+    uint32_t bl_cap, max_steps;
+};
+
+struct SmallShared {
+    TravCtl c;
+    uint32_t vin[kSmallCap];                   // the superstep's input
+    SmallIndex ix;                             // its edges
+    uint32_t v[kSmallCap], obeg[kSmallCap];    // the next one's
+    uint16_t odeg[kSmallCap];                  // (at most kSmallEdges + 1: too many either way)
+    uint32_t seen[kSmallHash];                 // vertices queued by this superstep
+    uint32_t n;
+};
+
+// The mode of superstep c is one the small path runs (its size allowing).
+__device__ __forceinline__ bool sssp_small_ok(const TravCtl &c) {
+    if (c.done) return false;
+    if (c.mode == kModeRelax || c.mode == kModeRelaxAll) return c.qsize[c.cur] <= kSmallCap;
+    if (c.mode == kModeSplit || c.mode == kModeSubSplit) return c.far_size[c.far_cur] <= kSmallFar;
+    return false;
+}
+
+__device__ __forceinline__ uint2 small_range(const SsspSmall &x, bool all, uint32_t v) {
+    if (all) return make_uint2(__ldg(&x.rowptr[v]), __ldg(&x.rowptr[v + 1]));
+    return __ldg(&x.lr[v]);
+}
+
+// Entry pos of the near queue: in shared memory with its row range, or past
+// its capacity in the global queue.
+__device__ __forceinline__ void small_put(uint32_t pos, uint32_t v, uint2 r, uint32_t *q,
+                                          SmallShared &sh) {
+    if (pos < kSmallCap) {
+        sh.v[pos] = v;
+        sh.obeg[pos] = r.x;
+        sh.odeg[pos] = (uint16_t)min(r.y - r.x, kSmallEdges + 1);
+    } else {
+        q[pos] = v;
+    }
+}
+
+// What a relax superstep's edges need besides the shared state.
+struct SmallStep {
+    uint32_t threshold, *fbits, *qout, *far, *far_size;
+    bool all;
+};
+
+// Edges base .. base + 1024 N - 1 of the input in sh, N per thread in flight.
+// A vertex whose distance this superstep lowers below the threshold is queued;
+// a small hash of the vertices queued so far drops most repeats (a repeat only
+// costs its edges once more).  The far pile is deduplicated by its marks, as in
+// the kernel chain.
+template <int N>
+__device__ __forceinline__ void small_edges(const SsspSmall &x, const SmallStep &a, uint32_t base,
+                                            uint32_t total, uint32_t *dist, uint32_t &fmin,
+                                            SmallShared &sh) {
+    // each stage issues all its loads or atomics before any result is used
+    uint32_t at[N], src[N], du[N], old[N], nd[N], pos[N];
+    uint2 e[N], r[N];
+    bool act[N], near[N], far[N];
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        const uint32_t k = base + j * kSmallThreads + threadIdx.x;
+        act[j] = k < total;
+        at[j] = 0;
+        src[j] = 0;
+        if (act[j]) {
+            const uint32_t lo = sh.ix.owner(k);
+            at[j] = sh.ix.beg[lo] + (k - sh.ix.off[lo]);
+            src[j] = sh.vin[lo];
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        e[j] = act[j] ? __ldg(&x.cw[at[j]]) : make_uint2(0u, 0u);
+        du[j] = act[j] ? __ldcg(&dist[src[j]]) : 0u;
+    }
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        nd[j] = du[j] + e[j].y;
+        if (nd[j] < du[j] || nd[j] > (uint32_t)kInf) nd[j] = (uint32_t)kInf;   // saturate
+        old[j] = act[j] ? atomicMin(&dist[e[j].x], nd[j]) : 0u;
+        r[j] = act[j] && nd[j] < a.threshold ? small_range(x, a.all, e[j].x) : make_uint2(0u, 0u);
+    }
+    bool anyfar = false;
+    const uint32_t (&v)[N] = at;
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        at[j] = e[j].x;
+        const bool low = old[j] > nd[j];   // this edge lowered the distance
+        near[j] = low && nd[j] < a.threshold;
+        far[j] = low && nd[j] >= a.threshold;
+        anyfar |= far[j];
+    }
+#pragma unroll
+    for (int j = 0; j < N; j++)
+        if (near[j]) near[j] = atomicExch(&sh.seen[v[j] % kSmallHash], v[j]) != v[j];
+    small_place(near, &sh.n, pos);
+#pragma unroll
+    for (int j = 0; j < N; j++)
+        if (near[j]) small_put(pos[j], v[j], r[j], a.qout, sh);
+    if (__any_sync(0xffffffffu, anyfar)) {
+#pragma unroll
+        for (int j = 0; j < N; j++)
+            old[j] = far[j] ? atomicOr(&a.fbits[v[j] >> 5], 1u << (v[j] & 31)) : 0u;
+#pragma unroll
+        for (int j = 0; j < N; j++)
+            if (far[j]) {
+                fmin = min(fmin, nd[j]);
+                far[j] = !((old[j] >> (v[j] & 31)) & 1u);
+            }
+        small_place(far, a.far_size, pos);
+#pragma unroll
+        for (int j = 0; j < N; j++)
+            if (far[j]) a.far[pos[j]] = v[j];
+    }
+}
+
+// Relax supersteps from the near queue (n vertices in sh.v / obeg / odeg)
+// until it is empty or does not fit.  Between two of them only the queue and
+// the counters move on, kept by every thread alike; the end step of the one
+// that empties the queue is left to the caller (returns true).
+__device__ bool small_relax(const SsspSmall &x, uint32_t n, uint32_t *dist, SmallShared &sh) {
+    const uint32_t t = threadIdx.x;
+    SmallStep a;
+    a.all = sh.c.mode == kModeRelaxAll;
+    a.threshold = sh.c.threshold;
+    a.fbits = (sh.c.epoch & 1) ? x.fm.m1 : x.fm.m0;
+    a.far = sh.c.far_cur ? x.far1 : x.far0;
+    a.far_size = &sh.c.far_size[sh.c.far_cur];
+    uint32_t cur = sh.c.cur, steps = sh.c.steps, bl_size = sh.c.bl_size;
+    bool bl_over = sh.c.bl_over != 0;
+    const uint32_t steps0 = steps;
+    uint32_t fmin = 0xffffffffu;
+    unsigned long long relaxed = 0;
+    bool drained = false;
+    for (;;) {
+        const uint32_t total = sh.ix.number(
+            n, steps, [&](uint32_t i) { return (uint32_t)sh.odeg[i]; },
+            [&](uint32_t i) { return sh.obeg[i]; });
+        if (total > kSmallEdges) break;
+        // the bucket list, under the end step's capacity test
+        const bool list = !a.all && !bl_over && (uint64_t)bl_size + n <= x.bl_cap;
+        for (uint32_t i = t; i < n; i += kSmallThreads) {
+            sh.vin[i] = sh.v[i];
+            if (list) x.blist[bl_size + i] = sh.v[i];
+        }
+        sh.seen[t] = 0xffffffffu;
+        if (t == 0) sh.n = 0;
+        a.qout = cur ? x.q0 : x.q1;
+        __syncthreads();
+        if (total <= kSmallThreads)
+            small_edges<1>(x, a, 0, total, dist, fmin, sh);
+        else if (total <= 2 * kSmallThreads)
+            small_edges<2>(x, a, 0, total, dist, fmin, sh);
+        else
+            for (uint32_t base = 0; base < total; base += kSmallThreads * kSmallItems)
+                small_edges<kSmallItems>(x, a, base, total, dist, fmin, sh);
+        relaxed += total;
+        __syncthreads();
+        const uint32_t next = sh.n;
+        if (next == 0) {
+            drained = true;
+            break;
+        }
+        if (!a.all && !bl_over) {
+            if ((uint64_t)bl_size + n <= x.bl_cap)
+                bl_size += n;
+            else
+                bl_over = true;
+        }
+        cur ^= 1;
+        steps++;
+        n = next;
+        if (n > kSmallCap || steps > x.max_steps) break;
+    }
+    const uint32_t m = __reduce_min_sync(0xffffffffu, fmin);
+    if (lane_id() == 0 && m != 0xffffffffu) atomicMin(&sh.c.far_min, m);
+    if (t == 0) {
+        sh.c.edges_relaxed += relaxed;
+        sh.c.cur = cur;
+        sh.c.qsize[cur] = n;
+        sh.c.qsize[cur ^ 1] = 0;
+        sh.c.steps = steps;
+        sh.c.bl_size = bl_size;
+        sh.c.bl_over = bl_over;
+        if (steps > x.max_steps && steps != steps0) {
+            sh.c.err = 2;
+            sh.c.done = 1;
+        }
+    }
+    __syncthreads();
+    return drained;
+}
+
+// One split of the far pile (as sssp_split): entries under the old threshold
+// are dropped, those under the new one are queued, the rest move on.
+__device__ void small_split(const SsspSmall &x, const uint32_t *dist, SmallShared &sh) {
+    const uint32_t fc = sh.c.far_cur, n = sh.c.far_size[fc];
+    const uint32_t *fin = fc ? x.far1 : x.far0;
+    uint32_t *fout = fc ? x.far0 : x.far1;
+    uint32_t *qn = sh.c.cur ? x.q1 : x.q0;
+    const uint32_t lo = sh.c.split_lo, hi = sh.c.threshold;
+    uint32_t *fcur = (sh.c.epoch & 1) ? x.fm.m1 : x.fm.m0;
+    uint32_t *fnext = (sh.c.epoch & 1) ? x.fm.m0 : x.fm.m1;
+    const bool all = sh.c.all_edges != 0;
+    if (threadIdx.x == 0) sh.n = 0;
+    __syncthreads();
+    uint32_t fmin = 0xffffffffu;
+    for (uint32_t base = 0; base < n; base += kSmallThreads * kSmallItems) {
+        uint32_t v[kSmallItems], d[kSmallItems], pos[kSmallItems];
+        uint2 r[kSmallItems];
+        bool near[kSmallItems], stay[kSmallItems];
+#pragma unroll
+        for (int j = 0; j < kSmallItems; j++) {
+            const uint32_t i = base + j * kSmallThreads + threadIdx.x;
+            v[j] = i < n ? __ldcg(&fin[i]) : 0xffffffffu;
+        }
+#pragma unroll
+        for (int j = 0; j < kSmallItems; j++) {
+            d[j] = 0;
+            r[j] = make_uint2(0u, 0u);
+            if (v[j] != 0xffffffffu) {
+                atomicAnd(&fcur[v[j] >> 5], ~(1u << (v[j] & 31)));   // this pile is consumed
+                d[j] = __ldcg(&dist[v[j]]);
+                r[j] = small_range(x, all, v[j]);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kSmallItems; j++) {
+            const bool live = v[j] != 0xffffffffu && d[j] >= lo;
+            near[j] = live && d[j] < hi;
+            stay[j] = live && d[j] >= hi;
+            if (stay[j]) {
+                atomicOr(&fnext[v[j] >> 5], 1u << (v[j] & 31));
+                fmin = min(fmin, d[j]);
+            }
+        }
+        small_place(near, &sh.n, pos);
+#pragma unroll
+        for (int j = 0; j < kSmallItems; j++)
+            if (near[j]) small_put(pos[j], v[j], r[j], qn, sh);
+        small_place(stay, &sh.c.far_size[fc ^ 1], pos);
+#pragma unroll
+        for (int j = 0; j < kSmallItems; j++)
+            if (stay[j]) fout[pos[j]] = v[j];
+    }
+    const uint32_t m = __reduce_min_sync(0xffffffffu, fmin);
+    if (lane_id() == 0 && m != 0xffffffffu) atomicMin(&sh.c.far_min, m);
+    __syncthreads();
+    if (threadIdx.x == 0) sh.c.qsize[sh.c.cur] = sh.n;
+}
+
+// The near queue for the kernel chain: each vertex once, in the global queue,
+// with its near mark set (the chain's next superstep clears it).
+__device__ void small_leave(const SsspSmall &x, SmallShared &sh) {
+    const uint32_t n = sh.c.qsize[sh.c.cur];
+    if (n == 0) return;
+    const uint32_t *qin = sh.c.cur ? x.q1 : x.q0;
+    uint32_t *qout = sh.c.cur ? x.q0 : x.q1;
+    uint32_t *nmark = (sh.c.steps & 1) ? x.nmark1 : x.nmark0;
+    if (threadIdx.x == 0) sh.n = 0;
+    __syncthreads();
+    for (uint32_t base = 0; base < n; base += kSmallThreads) {
+        const uint32_t i = base + threadIdx.x;
+        uint32_t v = 0, pos[1];
+        bool fresh[1] = {false};
+        if (i < n) {
+            v = i < kSmallCap ? sh.v[i] : __ldcg(&qin[i]);
+            const uint32_t bit = 1u << (v & 31);
+            fresh[0] = !(atomicOr(&nmark[v >> 5], bit) & bit);
+        }
+        small_place(fresh, &sh.n, pos);
+        if (fresh[0]) qout[pos[0]] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        sh.c.qsize[sh.c.cur] = 0;
+        sh.c.cur ^= 1;
+        sh.c.qsize[sh.c.cur] = sh.n;
+    }
+    __syncthreads();
+}
+
+// Whole CTA: supersteps from the control block's state (its mode chosen) until
+// one does not fit or the run is over.  sh.c holds the control block.
+__device__ void sssp_small(const SsspSmall &x, cudaGraphConditionalHandle h, SmallShared &sh) {
+    uint32_t *dist = static_cast<uint32_t *>(sh.c.vdata);
+    bool loaded = false;   // the near queue is in shared memory (the same in every thread)
+    while (sssp_small_ok(sh.c)) {
+        if (sh.c.mode == kModeSplit || sh.c.mode == kModeSubSplit) {
+            small_split(x, dist, sh);
+            loaded = true;
+        } else {
+            const uint32_t n = sh.c.qsize[sh.c.cur];
+            if (!loaded) {   // queued by the kernel chain: its near marks are cleared here
+                const uint32_t *q = sh.c.cur ? x.q1 : x.q0;
+                uint32_t *nprev = (sh.c.steps & 1) ? x.nmark1 : x.nmark0;
+                const bool all = sh.c.mode == kModeRelaxAll;
+                for (uint32_t i = threadIdx.x; i < n; i += kSmallThreads) {
+                    const uint32_t v = __ldcg(&q[i]);
+                    atomicAnd(&nprev[v >> 5], ~(1u << (v & 31)));
+                    small_put(i, v, small_range(x, all, v), nullptr, sh);
+                }
+                __syncthreads();
+                loaded = true;
+            }
+            if (!small_relax(x, n, dist, sh)) break;
+        }
+        if (threadIdx.x == 0) sssp_end_step(&sh.c, h, 0, x.max_steps, x.bl_cap);
+        __syncthreads();
+    }
+    if (loaded && !sh.c.done) small_leave(x, sh);
+}
+
+// Start of a run: control block, source, and the supersteps that fit one CTA.
+struct SsspStart {
+    uint32_t src, delta, sub, sub_buckets, tail_width, route, direct_min;
+    const uint32_t *newid;      // relabelled run: the source's new id
+    uint32_t *dist;
+    unsigned long long *red;    // cleared here when set
+};
+
+__global__ void __launch_bounds__(kSmallThreads)
+k_sssp_init(TravCtl *c, SsspStart a, SsspSmall x, cudaGraphConditionalHandle h, int use_cond) {
+    __shared__ SmallShared sh;
+    if (threadIdx.x == 0) {
+        const uint32_t src = a.newid ? a.newid[a.src] : a.src;
+        TravCtl t = {};
+        t.qsize[0] = 1;
+        t.vdata = a.dist;
+        t.delta = a.delta;
+        t.bucket_end = a.delta;
+        t.sub_width = a.sub < a.delta ? a.sub : 0;
+        t.sub_buckets = a.sub_buckets;
+        t.heavy_index = 0;
+        t.tail_width = a.tail_width > a.delta ? a.tail_width : 0;
+        t.all_edges = 0;
+        t.route = t.tail_width != 0 && a.route;
+        t.direct_min = t.route ? a.direct_min : 0;
+        t.threshold = (t.sub_width && a.sub_buckets > 0) ? t.sub_width : a.delta;
+        t.epoch = 1;
+        t.far_min = 0xffffffffu;
+        t.heavy_done = 0;
+        t.bucket_lo = 0;
+        a.dist[src] = 0;
+        x.q0[0] = src;
+        sssp_begin(&t);
+        sh.c = t;
+        if (a.red) {
+            a.red[0] = 0;
+            a.red[1] = 0;
+        }
+    }
+    __syncthreads();
+    sssp_small(x, h, sh);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        *c = sh.c;
+        if (use_cond) cudaGraphSetConditional(h, sh.c.done ? 0u : 1u);
+    }
+}
+
+__global__ void __launch_bounds__(kSmallThreads)
+k_sssp_end(TravCtl *c, cudaGraphConditionalHandle h, int use_cond, SsspSmall x) {
+    __shared__ SmallShared sh;
+    if (threadIdx.x == 0) {
+        sh.c = *c;
+        sssp_end_step(&sh.c, h, 0, x.max_steps, x.bl_cap);
+    }
+    __syncthreads();
+    sssp_small(x, h, sh);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        *c = sh.c;
+        if (use_cond) cudaGraphSetConditional(h, sh.c.done ? 0u : 1u);
+    }
+}
+
+// Before a run: unreached distances and empty mark bitmaps.
+__global__ void __launch_bounds__(kBlock)
+k_sssp_clear(uint32_t *__restrict__ dist, uint32_t V, uint4 *__restrict__ marks, uint64_t nm) {
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    for (uint64_t i = tid; i < nm; i += stride) marks[i] = make_uint4(0, 0, 0, 0);
+    if (reinterpret_cast<uintptr_t>(dist) & 15) {   // caller buffer not 16-byte aligned
+        for (uint64_t i = tid; i < V; i += stride) dist[i] = (uint32_t)kInf;
+        return;
+    }
+    const uint64_t n4 = V / 4;
+    uint4 *d4 = reinterpret_cast<uint4 *>(dist);
+    const uint4 inf4 = make_uint4(kInf, kInf, kInf, kInf);
+    for (uint64_t i = tid; i < n4; i += stride) d4[i] = inf4;
+    for (uint64_t i = n4 * 4 + tid; i < V; i += stride) dist[i] = (uint32_t)kInf;
 }
 
 // The superstep's dense pass: collect the settled bucket (heavy mode), pull
@@ -1121,6 +1511,29 @@ static int sssp_partition(olv_graph *g) {
     return OLV_OK;
 }
 
+static SsspSmall sssp_small_args(olv_graph *g) {
+    Workspace &ws = g->ws;
+    const size_t words = mark_words(g->V);
+    uint32_t *mk = ws.mark.as<uint32_t>();
+    SsspSmall x;
+    x.lr = ws.sssp_lr.as<uint2>();
+    x.rowptr = sssp_csr(g).rowptr;
+    x.cw = ws.sssp_cw.as<uint2>();
+    x.q0 = ws.q0.as<uint32_t>();
+    x.q1 = ws.q1.as<uint32_t>();
+    x.far0 = ws.far0.as<uint32_t>();
+    x.far1 = ws.far1.as<uint32_t>();
+    x.nmark0 = mk;
+    x.nmark1 = mk + words;
+    x.fm.m0 = mk + 2 * words;
+    x.fm.m1 = mk + 3 * words;
+    x.blist = ws.blist.as<uint32_t>();
+    x.bl_cap = g->V;
+    // a correct run needs far fewer supersteps; the bound only stops a runaway loop
+    x.max_steps = (uint32_t)std::min<uint64_t>(3ULL * g->V + 1000, 0xfffffff0ULL);
+    return x;
+}
+
 template <class Sink>
 static int sssp_superstep(olv_graph *g, Sink &&sink, cudaGraphConditionalHandle h,
                           int use_cond) {
@@ -1150,9 +1563,6 @@ static int sssp_superstep(olv_graph *g, Sink &&sink, cudaGraphConditionalHandle 
     fm.m0 = op.fmark0;
     fm.m1 = op.fmark1;
     uint32_t *q0 = a.q0, *q1 = a.q1, *far0 = a.far0, *far1 = a.far1;
-    // a correct run needs far fewer supersteps; the bound only stops a runaway loop
-    uint32_t max_steps = (uint32_t)(3ULL * g->V + 1000 > 0xfffffff0ULL ? 0xfffffff0ULL
-                                                                    : 3ULL * g->V + 1000);
     // the relax kernel for the tuned sources per thread (1, 2, 4 or 8)
     const uint32_t spt = g->tune.sssp_spt;
     const void *chunks = spt == 8   ? (const void *)k_advance_chunks<SsspOp, 8>
@@ -1192,28 +1602,46 @@ static int sssp_superstep(olv_graph *g, Sink &&sink, cudaGraphConditionalHandle 
     // relax supersteps cost less and the pull's chunks stay as balanced
     const int nba = 2 * g->num_sms;
     OLV_TRY(sink((const void *)k_sssp_aux, dim3(nba), dim3(kBlock), a_aux));
-    uint32_t bl_cap = x.bl_cap;
+    SsspSmall sm = sssp_small_args(g);
     // the end step runs in the pieces kernel's last CTA, or as its own launch
     op.end_h = h;
     op.end_fused = g->tune.sssp_fuse_end;
     op.end_use_cond = use_cond;
-    op.end_max_steps = max_steps;
-    op.end_bl_cap = bl_cap;
+    op.end_max_steps = sm.max_steps;
+    op.end_bl_cap = sm.bl_cap;
     void *a_adv[] = {&a, &op};
     OLV_TRY(sink(chunks, dim3(nb), dim3(kBlock), a_adv));
     OLV_TRY(sink((const void *)k_advance_pieces<SsspOp>, dim3(nb), dim3(kBlock), a_adv));
     if (!op.end_fused) {
-        void *a_end[] = {&ctl, &h, &use_cond, &max_steps, &bl_cap};
-        OLV_TRY(sink((const void *)k_sssp_end, dim3(1), dim3(1), a_end));
+        void *a_end[] = {&ctl, &h, &use_cond, &sm};
+        OLV_TRY(sink((const void *)k_sssp_end, dim3(1), dim3(kSmallThreads), a_end));
     }
     return OLV_OK;
 }
 
-static int sssp_graph(olv_graph *g) {
-    if (g->sssp_graph && g->sssp_graph->ready) return OLV_OK;
+// Arguments of k_sssp_init for one run (the kernel's parameters by address).
+struct SsspInitArgs {
+    TravCtl *ctl;
+    SsspStart start;
+    SsspSmall small;
+    cudaGraphConditionalHandle h = 0;
+    int use_cond = 0;
+    void *p[5] = {&ctl, &start, &small, &h, &use_cond};
+};
+
+static int sssp_graph(olv_graph *g, SsspInitArgs &init) {
     if (!g->sssp_graph) g->sssp_graph = new WhileGraph();
     WhileGraph &wg = *g->sssp_graph;
-    OLV_TRY(wg.begin());
+    const void *fn = (const void *)k_sssp_init;
+    init.use_cond = 1;
+    if (wg.ready) {   // the run's own source and output
+        init.h = wg.handle;
+        return wg.set_root(fn, dim3(1), dim3(kSmallThreads), init.p);
+    }
+    OLV_TRY(wg.create());
+    init.h = wg.handle;
+    OLV_TRY(wg.add_root(fn, dim3(1), dim3(kSmallThreads), init.p));
+    OLV_TRY(wg.open_loop());
     auto sink = [&](const void *f, dim3 gr, dim3 bl, void **args) { return wg.add(f, gr, bl, args); };
     OLV_TRY(sssp_superstep(g, sink, wg.handle, 1));
     return wg.finish();
@@ -1229,7 +1657,7 @@ int sssp_workspace(olv_graph *g) {
     return OLV_OK;
 }
 
-// red (device, [2], zeroed; or null): reached out-edges and vertices, summed
+// red (device, [2]; or null): reached out-edges and vertices, summed
 // by the final pass when the run is renumbered; *red_done says whether it was.
 int run_sssp_device(olv_graph *g, uint32_t src, uint32_t *dist_dev, unsigned long long *red,
                     bool *red_done) {
@@ -1239,15 +1667,19 @@ int run_sssp_device(olv_graph *g, uint32_t src, uint32_t *dist_dev, unsigned lon
     TravCtl *ctl = g->ws.ctl.as<TravCtl>();
     const SsspCsr R = sssp_csr(g);
     uint32_t *dist = R.dist ? R.dist : dist_dev;   // renumbered run: internal distances
-    OLV_CUDA(cudaMemsetAsync(g->ws.mark.p, 0, kMarks * mark_words(g->V) * 4, s));
-    k_fill_i32<<<g->num_sms * 8, kBlock, 0, s>>>((int32_t *)dist, g->V, kInf);
-    k_sssp_init<<<1, 1, 0, s>>>(ctl, dist, g->ws.q0.as<uint32_t>(), src, sssp_delta(g),
-                                g->tune.sssp_sub, g->tune.sssp_sub_buckets,
-                                g->tune.sssp_tail_delta, g->tune.sssp_route,
-                                g->tune.sssp_pull_direct && g->tune.sssp_pull && g->ws.sssp_crw.p
-                                    ? std::max<uint32_t>(1u, g->V / 16) : 0u,
-                                R.newid);
+    const uint64_t nm = kMarks * mark_words(g->V) / 4;   // mark words in 16-byte units
+    const int clear_blocks =
+        (int)std::min<uint64_t>((uint64_t)g->num_sms * 8, (g->V / 4 + nm) / kBlock + 1);
+    k_sssp_clear<<<clear_blocks, kBlock, 0, s>>>(dist, g->V, g->ws.mark.as<uint4>(), nm);
     OLV_CUDA(cudaGetLastError());
+    SsspInitArgs init;
+    init.ctl = ctl;
+    init.start = SsspStart{src, sssp_delta(g), g->tune.sssp_sub, g->tune.sssp_sub_buckets,
+                           g->tune.sssp_tail_delta, (uint32_t)g->tune.sssp_route,
+                           g->tune.sssp_pull_direct && g->tune.sssp_pull && g->ws.sssp_crw.p
+                               ? std::max<uint32_t>(1u, g->V / 16) : 0u,
+                           R.newid, dist, red};
+    init.small = sssp_small_args(g);
     auto finish = [&]() -> int {
         if (R.dist) {
             k_sssp_unrelabel<<<g->num_sms * 8, kBlock, 0, s>>>(R.dist, R.newid, g->V, dist_dev,
@@ -1258,12 +1690,15 @@ int run_sssp_device(olv_graph *g, uint32_t src, uint32_t *dist_dev, unsigned lon
         return OLV_OK;
     };
     if (g->tune.use_graphs) {
-        if (sssp_graph(g) == OLV_OK) {
+        if (sssp_graph(g, init) == OLV_OK) {
             OLV_TRY(g->sssp_graph->launch(s));
             return finish();
         }
         g->tune.use_graphs = 0;
+        init.h = 0;
+        init.use_cond = 0;
     }
+    OLV_CUDA(cudaLaunchKernel((const void *)k_sssp_init, dim3(1), dim3(kSmallThreads), init.p, 0, s));
     auto launch = [&](const void *f, dim3 gr, dim3 bl, void **args) {
         OLV_CUDA(cudaLaunchKernel(f, gr, bl, args, 0, s));
         return OLV_OK;
@@ -1292,8 +1727,7 @@ extern "C" int olv_sssp(olv_graph *g, uint32_t src, uint32_t *dist_out, olv_stat
     cudaStream_t s = g->stream;
     unsigned long long *red_dev = nullptr;
     if (st) {
-        OLV_TRY(g->ws.tmp.ensure(16));
-        OLV_CUDA(cudaMemsetAsync(g->ws.tmp.p, 0, 16, s));
+        OLV_TRY(g->ws.tmp.ensure(16));   // cleared at the start of the run
         red_dev = g->ws.tmp.as<unsigned long long>();
     }
     bool red_done = false;

@@ -62,3 +62,29 @@ def test_bfs_layers(ob, shape, graphs):
             np.testing.assert_array_equal(g.bfs(s), ref)
             assert g.last_stats.edges_traversed == e_ref
             assert g.last_stats.iterations == len(SHAPES[shape][0])
+
+
+@pytest.mark.parametrize("wmax", [1, 255, 5000])
+@pytest.mark.parametrize("shape", range(len(SHAPES)))
+def test_sssp_layers(ob, shape, wmax):
+    rp, cl, src = layered(*SHAPES[shape], seed=shape + 50)
+    w = np.random.default_rng(wmax).integers(1, wmax + 1, len(cl)).astype(np.uint32)
+    ref, e_ref, _, nset = oracle.dijkstra(rp, cl, w, src)
+    with ob.Graph.from_csr(rp, cl, w) as g:
+        for kw in ({}, {"use_graphs": 0}, {"sssp_tail_delta": 0}, {"sssp_relabel": 0},
+                   {"sssp_sub": 4}, {"sssp_pull": 0}):
+            base = g.tune()
+            g.tune(**kw)
+            np.testing.assert_array_equal(g.sssp(src), ref, err_msg=str(kw))
+            st = g.last_stats
+            assert st.edges_traversed == e_ref and st.vertices_reached == nset
+            g.tune(**{k: base[k] for k in kw})
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 1), (3, 700), (90, 101)])
+def test_sssp_grid(ob, rows, cols):
+    rp, cl = oracle.grid_csr(rows, cols)
+    w = np.random.default_rng(rows).integers(0, 256, len(cl)).astype(np.uint32)
+    with ob.Graph.from_csr(rp, cl, w) as g:
+        for s in (0, rows * cols // 2):
+            np.testing.assert_array_equal(g.sssp(s), oracle.dijkstra(rp, cl, w, s)[0])
