@@ -80,3 +80,27 @@ def test_ppr_bad_arguments(ob):
             g.ppr(np.array([16], np.uint32))
         with pytest.raises(ob.OliveError):
             g.ppr(np.array([], np.uint32))
+
+
+@pytest.mark.parametrize("longest", [1, 7, 8, 9, 255, 256, 257, 511, 513, 4000])
+def test_ppr_row_lengths(ob, longest):
+    """Rows on both sides of the eight-entry rounds and of the 256-entry
+    segments, seeds on rows without in-edges (with and without out-edges), and
+    two damping factors on one handle."""
+    rng = np.random.default_rng(longest)
+    V = 5003
+    din = np.zeros(V, np.int64)
+    din[:40] = longest
+    din[40:2000] = rng.integers(0, 20, 1960)       # the rest have no in-edges
+    dst = np.repeat(np.arange(V), din)
+    src = rng.integers(0, 3000, len(dst))           # vertices from 3000 on: no out-edges
+    o = np.argsort(src, kind="stable")
+    rp = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=V))]).astype(np.uint32)
+    cl = dst[o].astype(np.uint32)
+    with ob.Graph.from_csr(rp, cl) as g:
+        seeds = np.array([0, 2500, 2500, 4000, int(src[0]), 39] + list(range(50, 76)), np.uint32)
+        for alpha in (0.85, 0.5):
+            for K in (32, 6):
+                out = g.ppr(seeds[:K], alpha, 12, 0.0)
+                ref, _ = oracle.ppr(rp, cl, seeds[:K], alpha, 12, 0.0)
+                check(out, ref)
