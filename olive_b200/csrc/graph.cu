@@ -481,12 +481,8 @@ int olv_graph_copy_csr(const olv_graph *g, uint32_t *rowptr, uint32_t *col, void
 int olv_graph_set_weights_f32(olv_graph *g, const float *w) {
     OLV_CHECK_ARG(g && (w || g->E == 0), "olv_graph_set_weights_f32: null pointer");
     OLV_TRY(copy_in(g->w, w, g->E * 4, g->stream));
+    // no CSC copy: only SSSP reads one, and its weights are uint32
     g->weight_type = OLV_W_F32;
-    OLV_TRY(g->csc_w.ensure(g->E * 4 + 16));
-    if (g->E)
-        k_gather<uint32_t><<<grid_for(g->E, g->num_sms), kBlock, 0, g->stream>>>(
-            g->w.as<uint32_t>(), g->csc_eid.as<uint32_t>(), g->E, g->csc_w.as<uint32_t>());
-    OLV_CUDA(cudaGetLastError());
     return OLV_OK;
 }
 

@@ -10,7 +10,7 @@
 //     at the front of every per-vertex array, so their lines stay in L1/L2;
 //   * the per-row inputs and outputs are read and written as contiguous runs.
 // Rows longer than kTileLong are cut into kTileSeg-entry segments summed by
-// k_row_segments (olv_rowsum.cuh) and folded in segment order.
+// k_row_segments and folded in segment order.
 //
 // Every sum has a fixed evaluation order: lane j of a row's group adds the
 // row's entries j, j+G, j+2G, ... in order with compensated (two-sum) FP32
@@ -18,18 +18,16 @@
 // take tiles by a fixed stride over a fixed grid, so the FP64 partials the
 // row updates produce are also summed in a fixed order.
 //
-// The Op interface is that of olv_rowsum.cuh; row ids are the new ids.
-//
-// A plan can also keep the neighbour ids (relabel = false): only the rows are
-// reordered, `pos` maps each entry to its position in the original structure
-// (to permute per-entry values such as edge weights), and PermOp hands the
-// original row id to an Op whose per-vertex arrays stay in the original
-// order.
+// An Op supplies (row ids are the new ids):
+//   void begin()                                per-launch setup (ping-pong choice)
+//   float term(uint32_t e, uint32_t j)          value of entry e with neighbour j
+//   struct Row; Row row(uint32_t v)             per-row inputs of the update
+//   void finish(uint32_t v, float s, float c, const Row &r, double &res, double &aux)
+//                                               consume the row sum s + c; res and aux
+//                                               are FP64 partials
+//   const uint32_t *done                        the kernels return when *done
 #pragma once
-#include <algorithm>
-#include <vector>
-
-#include "olv_rowsum.cuh"
+#include "olv_rowsolve.cuh"
 
 namespace olv {
 
@@ -46,6 +44,7 @@ constexpr uint32_t kTileSeg = OLV_TILE_SEG;   // entries per segment of a long r
 #endif
 constexpr int kTileU = OLV_TILE_U;     // entries per lane per round (loads in flight)
 constexpr int kTileMinBlocks = OLV_TILE_MINB;   // resident CTAs per SM of the tile pass
+constexpr int kStrips = 8;             // 32-entry strips per warp with loads in flight (segments)
 constexpr uint32_t kNoSeg = 0xffffffu;
 constexpr uint32_t kTileCTAs = 148 * kTileMinBlocks;  // fixed grid of the tile pass
                                                       // (fixed partial order), one wave
@@ -58,142 +57,59 @@ struct TilePlan {
     DevBuf perm;      // new id -> old id
     DevBuf newid;     // old id -> new id
     DevBuf ptr;       // [n + 1] row offsets in the new order
-    DevBuf idx;       // neighbour (new or original) ids, rows in the new order
-    DevBuf pos;       // relabel = false: original position of every entry
+    DevBuf idx;       // neighbour ids, relabelled, rows in the new order
     DevBuf tiles, seg_range, segs, partials;
     uint32_t n = 0, ntiles = 0, nsegs = 0;
     void release() {
-        perm.release(); newid.release(); ptr.release(); idx.release(); pos.release();
-        tiles.release();
-        seg_range.release(); segs.release(); partials.release();
-    }
-};
-
-// idx[ptr[i] + k] = newid[old_idx[old_ptr[perm[i]] + k]] (or the original id
-// when newid is null, recording the entry's original position), one warp per
-// row.
-static __global__ void k_relabel_rows(const uint32_t *__restrict__ old_ptr,
-                               const uint32_t *__restrict__ old_idx,
-                               const uint32_t *__restrict__ perm, const uint32_t *__restrict__ newid,
-                               const uint32_t *__restrict__ ptr, uint32_t n,
-                               uint32_t *__restrict__ idx, uint32_t *__restrict__ pos) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t i = w; i < n; i += nw) {
-        const uint32_t v = perm[i];
-        const uint32_t b = old_ptr[v], e = old_ptr[v + 1], o = ptr[i];
-        for (uint32_t k = lane; k < e - b; k += 32) {
-            const uint32_t j = old_idx[b + k];
-            idx[o + k] = newid ? newid[j] : j;
-            if (pos) pos[o + k] = b + k;
-        }
-    }
-}
-
-// out[k] = in[pos[k]]: per-entry values in a plan's entry order.
-static __global__ void k_permute_entries(const float *__restrict__ in, const uint32_t *__restrict__ pos,
-                                  uint64_t n, float *__restrict__ out) {
-    for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < n;
-         k += (uint64_t)gridDim.x * blockDim.x)
-        out[k] = in[pos[k]];
-}
-
-// An Op over a row-reordered plan (relabel = false): row r of the plan is
-// vertex perm[r] of the Op's arrays; entry values come from arrays already
-// permuted to the plan's entry order.
-template <class Op>
-struct PermOp {
-    Op op;
-    const uint32_t *perm;
-    const uint32_t *done;
-    __device__ __forceinline__ void begin() { op.begin(); }
-    __device__ __forceinline__ float term(uint32_t e, uint32_t j) const { return op.term(e, j); }
-    struct Row {
-        typename Op::Row r;
-        uint32_t v;
-    };
-    __device__ __forceinline__ Row row(uint32_t r) const {
-        const uint32_t v = __ldg(&perm[r]);
-        return Row{op.row(v), v};
-    }
-    __device__ __forceinline__ void finish(uint32_t, float s, float c, const Row &q, double &res,
-                                           double &aux) const {
-        op.finish(q.v, s, c, q.r, res, aux);
+        perm.release(); newid.release(); ptr.release(); idx.release();
+        tiles.release(); seg_range.release(); segs.release(); partials.release();
     }
 };
 
 // Build the plan from a device row-offset array (n rows) and its neighbour
-// array.  The relabelling is a stable counting sort by row length
-// (descending), done on the host once per graph.
-// lanes_u: entries per lane per round the grouping aims at (rows get the
-// fewest lanes G = 1..32 with G * lanes_u >= row length); the autotuner's
-// "pr_tile_u".
-inline int build_tile_plan(const uint32_t *ptr_dev, const uint32_t *idx_dev, uint32_t n,
-                           cudaStream_t s, TilePlan &p, bool relabel = true,
-                           uint32_t lanes_u = kTileU) {
-    std::vector<uint32_t> cp((size_t)n + 1);
-    OLV_CUDA(cudaMemcpyAsync(cp.data(), ptr_dev, ((size_t)n + 1) * 4, cudaMemcpyDeviceToHost, s));
-    OLV_CUDA(cudaStreamSynchronize(s));
-    uint32_t maxd = 0;
-    for (uint32_t v = 0; v < n; v++) maxd = std::max(maxd, cp[v + 1] - cp[v]);
-    std::vector<uint32_t> start((size_t)maxd + 2, 0);
-    for (uint32_t v = 0; v < n; v++) start[maxd - (cp[v + 1] - cp[v]) + 1]++;
-    for (size_t d = 1; d < start.size(); d++) start[d] += start[d - 1];
-    std::vector<uint32_t> perm(n), newid(n), ptr((size_t)n + 1);
-    for (uint32_t v = 0; v < n; v++) {
-        const uint32_t i = start[maxd - (cp[v + 1] - cp[v])]++;
-        perm[i] = v;
-        newid[v] = i;
-    }
-    ptr[0] = 0;
-    for (uint32_t i = 0; i < n; i++) ptr[i + 1] = ptr[i] + (cp[perm[i] + 1] - cp[perm[i]]);
-    std::vector<uint2> tiles, ranges;
-    for (uint32_t i = 0; i < n;) {
-        const uint32_t d = ptr[i + 1] - ptr[i];
-        if (d > kTileLong) {
-            tiles.push_back(make_uint2(i, 5u | ((uint32_t)ranges.size() << 8)));
-            for (uint32_t x = ptr[i]; x < ptr[i + 1]; x += kTileSeg)
-                ranges.push_back(make_uint2(x, std::min(ptr[i + 1], x + kTileSeg)));
-            i++;
-            continue;
+// array (rowplan.cu).  lanes_u: entries per lane per round the grouping aims at
+// (rows get the fewest lanes G = 1..32 with G * lanes_u >= row length); the
+// autotuner's "pr_tile_u".
+int build_tile_plan(const uint32_t *ptr_dev, const uint32_t *idx_dev, uint32_t n, cudaStream_t s,
+                    TilePlan &p, uint32_t lanes_u = kTileU);
+
+// One warp per segment of a long row: each lane sums its entries (stride 32,
+// kStrips loads in flight) in order, then a fixed shuffle tree combines the
+// lanes.
+template <class Op>
+__global__ void __launch_bounds__(kBlock)
+k_row_segments(const uint32_t *__restrict__ idx, const uint2 *__restrict__ seg_range,
+               uint32_t nsegs, Op op, float2 *__restrict__ segs) {
+    if (*op.done) return;
+    op.begin();
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t w = (blockIdx.x * kBlock + threadIdx.x) >> 5;
+    if (w >= nsegs) return;   // whole warps only
+    const uint2 r = seg_range[w];
+    float s = 0.0f, c = 0.0f;
+    for (uint32_t base = r.x; base < r.y; base += 32 * kStrips) {
+        uint32_t j[kStrips];
+#pragma unroll
+        for (int q = 0; q < kStrips; q++) {
+            const uint32_t i = base + q * 32 + lane;
+            j[q] = i < r.y ? __ldg(&idx[i]) : 0u;
         }
-        uint32_t lg = 0;
-        while (lg < 5 && (1u << lg) * lanes_u < d) lg++;
-        tiles.push_back(make_uint2(i, lg | (kNoSeg << 8)));
-        i += 32u >> lg;
+        float x[kStrips];
+#pragma unroll
+        for (int q = 0; q < kStrips; q++) {
+            const uint32_t i = base + q * 32 + lane;
+            x[q] = i < r.y ? op.term(i, j[q]) : 0.0f;
+        }
+#pragma unroll
+        for (int q = 0; q < kStrips; q++) two_sum_acc(s, c, x[q]);
     }
-    if (ranges.size() >= kNoSeg) {
-        set_error("row plan: %zu segments exceed the tile format", ranges.size());
-        return OLV_ERR_LIMIT;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        const float s2 = __shfl_down_sync(0xffffffffu, s, o);
+        const float c2 = __shfl_down_sync(0xffffffffu, c, o);
+        pair_add(s, c, s2, c2);
     }
-    p.n = n;
-    p.ntiles = (uint32_t)tiles.size();
-    p.nsegs = (uint32_t)ranges.size();
-    const size_t E = ptr[n];
-    OLV_TRY(p.perm.ensure((size_t)n * 4 + 16));
-    OLV_TRY(p.newid.ensure((size_t)n * 4 + 16));
-    OLV_TRY(p.ptr.ensure(((size_t)n + 1) * 4));
-    OLV_TRY(p.idx.ensure(E * 4 + 16));
-    if (!relabel) OLV_TRY(p.pos.ensure(E * 4 + 16));
-    OLV_TRY(p.tiles.ensure(tiles.size() * 8 + 16));
-    OLV_TRY(p.seg_range.ensure(ranges.size() * 8 + 16));
-    OLV_TRY(p.segs.ensure(ranges.size() * 8 + 16));
-    OLV_TRY(p.partials.ensure((size_t)kTileCTAs * 16 + 16));
-    OLV_CUDA(cudaMemcpyAsync(p.perm.p, perm.data(), (size_t)n * 4, cudaMemcpyHostToDevice, s));
-    OLV_CUDA(cudaMemcpyAsync(p.newid.p, newid.data(), (size_t)n * 4, cudaMemcpyHostToDevice, s));
-    OLV_CUDA(cudaMemcpyAsync(p.ptr.p, ptr.data(), ((size_t)n + 1) * 4, cudaMemcpyHostToDevice, s));
-    OLV_CUDA(cudaMemcpyAsync(p.tiles.p, tiles.data(), tiles.size() * 8, cudaMemcpyHostToDevice, s));
-    if (!ranges.empty())
-        OLV_CUDA(cudaMemcpyAsync(p.seg_range.p, ranges.data(), ranges.size() * 8,
-                                 cudaMemcpyHostToDevice, s));
-    k_relabel_rows<<<1184, kBlock, 0, s>>>(ptr_dev, idx_dev, p.perm.as<uint32_t>(),
-                                          relabel ? p.newid.as<uint32_t>() : nullptr,
-                                          p.ptr.as<uint32_t>(), n, p.idx.as<uint32_t>(),
-                                          relabel ? nullptr : p.pos.as<uint32_t>());
-    OLV_CUDA(cudaGetLastError());
-    OLV_CUDA(cudaStreamSynchronize(s));
-    return OLV_OK;
+    if (lane == 0) segs[w] = make_float2(s, c);
 }
 
 template <class Op>

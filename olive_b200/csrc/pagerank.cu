@@ -10,31 +10,39 @@
 // every iteration (oliver.h:127) and copies all vertex values back to sum the
 // residual on the host (oliver.h:176-183).  Here:
 //   * the solve runs on a relabelled copy of the reverse graph (CSC): vertices
-//     renumbered by in-degree, longest rows first (olv_rowtiles.cuh), built
-//     once per graph.  Ranks, contributions r/outdeg and out-degrees live in
-//     the new order; the ranks are mapped back to the caller's ids once, at
-//     the end of the solve;
+//     renumbered by in-degree, longest rows first, built once per graph.  Ranks,
+//     contributions r/outdeg and out-degrees live in the new order; the ranks
+//     are mapped back to the caller's ids once, at the end of the solve;
 //   * each iteration is one pull pass over the in-edges: a group of 1..32
 //     lanes per row (by row length) sums the row's contributions in a fixed
 //     order with compensated (two-sum) FP32 arithmetic, so results do not
-//     depend on scheduling and carry ~1 rounding per vertex; rows longer than
-//     kTileLong are summed in fixed segments first;
+//     depend on scheduling and carry ~1 rounding per vertex;
 //   * the same pass writes the next iteration's contributions r/outdeg and
-//     per-CTA FP64 partial sums of |r' - r| and of the dangling mass;
-//   * a one-CTA kernel folds the partials in a fixed order (FP64), decides
-//     convergence on the device and sets the loop condition of the CUDA graph
-//     that runs all iterations.
+//     per-CTA FP64 partial sums of |r' - r| and of the dangling mass, which are
+//     folded in a fixed order and decide convergence on the device.
+//
+// Two ways to run the iterations.  All of them in one launch (olv_rowsolve.cuh)
+// where launches and the loop around them were most of the time (below
+// kPrSolveEdges edges), and on graphs without a segmented row of any size; else
+// an iteration is a tile pass and a one-CTA fold inside a CUDA graph
+// (olv_rowtiles.cuh), which reads the hubs' rows faster (no counts and fences
+// among the gathers).  Both measured, us for 20 iterations, tile pass / one
+// launch: RMAT-12 316 / 168, RMAT-16 457 / 363, RMAT-18 (3.9 M edges) 516 / 536,
+// RMAT-19 735 / 942, RMAT-21 2265 / 3070; uniform digraphs of 16 edges a vertex,
+// 2^16 vertices 343 / 264, 2^18 624 / 520, 2^21 3181 / 2912.
 #include <algorithm>
 #include <vector>
 
 #include "olive_b200/olv_advance.cuh"
 #include "olv_graphexec.cuh"
 #include "olv_internal.cuh"
+#include "olv_rowsolve.cuh"
 #include "olv_rowtiles.cuh"
 
 namespace olv {
 
-constexpr int kRedThreads = 1024;
+constexpr int kRedThreads = 1024;   // 32 warps: one more tree over them
+constexpr uint64_t kPrSolveEdges = 3u << 20;
 
 struct PrCtl {
     double base;        // (1-alpha)/N + alpha*d/N for the running iteration
@@ -47,6 +55,7 @@ struct PrCtl {
     double tol;
     double alpha;
     double inv_n;
+    float a_hi, a_lo;   // alpha as an unevaluated FP32 pair: the update carries FP64-level alpha
 };
 
 // r' = alpha * (s + c) + base, with alpha split into hi + lo FP32 parts.
@@ -56,23 +65,25 @@ __device__ __forceinline__ float pr_update(float s, float c, float a_hi, float a
 }
 
 // Row sums over in-edges of the contributions r[u]/outdeg(u); the row update
-// writes the rank, the next contribution and FP64 |r'-r| / dangling partials.
-struct PrOp {
+// writes the rank, the next contribution and FP64 |r'-r| / dangling partials
+// (olv_rowtiles.cuh).
+struct PrTileOp {
     const uint32_t *done;
     const PrCtl *ctl;
     const float *c0, *c1;
     float *rank;
     const uint32_t *outdeg;
-    float a_hi, a_lo;
     const float *cin;
     float *cout;
-    float base;
+    float a_hi, a_lo, base;
 
     __device__ __forceinline__ void begin() {
         const bool odd = ctl->iter & 1;
         cin = odd ? c1 : c0;
         cout = const_cast<float *>(odd ? c0 : c1);
         base = (float)ctl->base;
+        a_hi = ctl->a_hi;
+        a_lo = ctl->a_lo;
     }
     __device__ __forceinline__ float term(uint32_t, uint32_t j) const { return __ldg(&cin[j]); }
     struct Row {
@@ -94,33 +105,84 @@ struct PrOp {
     }
 };
 
+// The same for a whole solve in one launch (olv_rowsolve.cuh).
+struct PrOp {
+    static constexpr bool kGather = true, kWeighted = false, kStore = true;
+    float *c0, *c1;            // contributions, ping-pong
+    float *rank;
+    const uint32_t *outdeg;
+    const SolveCtl *ctl;
+    float a_hi, a_lo;
+    double alpha, inv_n;
+    int leak;
+    float rank0;
+    float base;
+    uint32_t odd;
+
+    // dangling mass of the start: an exact count, so that the first constant
+    // term does not depend on the order of atomics
+    __device__ __forceinline__ double first_aux() const {
+        return (double)ctl->count * (double)rank0;
+    }
+    __device__ __forceinline__ void begin(uint32_t it, double dang) {
+        odd = it & 1;
+        base = (float)((1.0 - alpha) * inv_n + (leak ? 0.0 : alpha * dang * inv_n));
+    }
+    __device__ __forceinline__ const float *in() const { return odd ? c1 : c0; }
+    __device__ __forceinline__ float *out() const { return odd ? c0 : c1; }
+    struct Row {
+        float old;       // rank before this iteration
+        uint32_t deg;    // out-degree
+    };
+    __device__ __forceinline__ Row row(uint32_t v) const { return Row{rank[v], __ldg(&outdeg[v])}; }
+    __device__ __forceinline__ float finish(uint32_t v, float s, float c, const Row &r, double &res,
+                                            double &dang) const {
+        const float nr = pr_update(s, c, a_hi, a_lo, base);
+        rank[v] = nr;
+        res += fabs((double)nr - (double)r.old);
+        if (r.deg) return __fdiv_rn(nr, (float)r.deg);
+        dang += (double)nr;
+        return 0.0f;
+    }
+};
+
 // Fold the per-CTA partials (fixed order), publish residual and the next
 // iteration's constant term, decide convergence.
 __global__ void __launch_bounds__(kRedThreads)
 k_pr_reduce(PrCtl *ctl, const double *__restrict__ partials, uint32_t nparts,
             cudaGraphConditionalHandle h, int use_cond) {
-    __shared__ double s[2][kRedThreads];
+    __shared__ double s[2][kRedThreads / 32];
     if (ctl->done) {
         if (use_cond && threadIdx.x == 0) cudaGraphSetConditional(h, 0u);
         return;
     }
     double a = 0, b = 0;
     for (uint32_t i = threadIdx.x; i < nparts; i += kRedThreads) {
-        a += partials[2 * i];
-        b += partials[2 * i + 1];
+        const double2 p = reinterpret_cast<const double2 *>(partials)[i];
+        a += p.x;
+        b += p.y;
     }
-    s[0][threadIdx.x] = a;
-    s[1][threadIdx.x] = b;
+    // a tree over each warp, then over the warps (one barrier)
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        a += __shfl_down_sync(0xffffffffu, a, o);
+        b += __shfl_down_sync(0xffffffffu, b, o);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        s[0][threadIdx.x >> 5] = a;
+        s[1][threadIdx.x >> 5] = b;
+    }
     __syncthreads();
-    for (int w = kRedThreads / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < (uint32_t)w) {
-            s[0][threadIdx.x] += s[0][threadIdx.x + w];
-            s[1][threadIdx.x] += s[1][threadIdx.x + w];
-        }
-        __syncthreads();
+    if (threadIdx.x >= 32) return;
+    a = s[0][threadIdx.x];
+    b = s[1][threadIdx.x];
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        a += __shfl_down_sync(0xffffffffu, a, o);
+        b += __shfl_down_sync(0xffffffffu, b, o);
     }
     if (threadIdx.x == 0) {
-        const double res = s[0][0], dang = s[1][0];
+        const double res = a, dang = b;
         ctl->residual = res;
         ctl->dangling = dang;
         ctl->iter++;
@@ -151,6 +213,8 @@ __global__ void k_pr_ctl_init(PrCtl *ctl, const unsigned long long *ndang, uint3
                               double alpha, uint32_t max_it, double tol, uint32_t leak) {
     PrCtl c = {};
     c.alpha = alpha;
+    c.a_hi = (float)alpha;
+    c.a_lo = (float)(alpha - (double)c.a_hi);
     c.inv_n = 1.0 / (double)V;
     c.tol = tol;
     c.max_it = max_it;
@@ -184,23 +248,31 @@ __global__ void k_pr_unpermute(const float *__restrict__ rank_new,
 
 // ------------------------------------------------------------------ host --
 struct PrPlan {
-    TilePlan tp;
+    bool solve = false;        // one launch for all iterations
+    SolvePlan sp;              // ... its structure,
+    TilePlan tp;               // or that of the tile pass
     DevBuf outdeg, contrib, rank, ctl, dang;   // outdeg, contrib, rank: new order
-    float a_hi = 0, a_lo = 0;
+    const uint32_t *perm() const { return (solve ? sp.perm : tp.perm).as<uint32_t>(); }
+    const uint32_t *newid() const { return (solve ? sp.newid : tp.newid).as<uint32_t>(); }
     ~PrPlan() {
-        tp.release(); outdeg.release(); contrib.release(); rank.release(); ctl.release();
-        dang.release();
+        sp.release(); tp.release(); outdeg.release(); contrib.release(); rank.release();
+        ctl.release(); dang.release();
     }
 };
 
 static int build_pr_plan(olv_graph *g, PrPlan &p) {
     const uint32_t V = g->V;
-    OLV_TRY(build_tile_plan(g->colptr.as<uint32_t>(), g->rowidx.as<uint32_t>(), V, g->stream,
-                            p.tp, true, g->tune.pr_tile_u));
+    p.solve = g->E < kPrSolveEdges || g->max_in_degree <= kRowLong;
+    if (p.solve)
+        OLV_TRY(build_solve_plan(g->colptr.as<uint32_t>(), g->rowidx.as<uint32_t>(), nullptr, V,
+                                 g->E, g->tune.pr_tile_u, false, g->num_sms, g->stream, p.sp));
+    else
+        OLV_TRY(build_tile_plan(g->colptr.as<uint32_t>(), g->rowidx.as<uint32_t>(), V, g->stream,
+                                p.tp, g->tune.pr_tile_u));
     OLV_TRY(p.outdeg.ensure((size_t)V * 4 + 16));
-    k_outdeg_perm<<<g->num_sms * 8, kBlock, 0, g->stream>>>(
-        g->rowptr.as<uint32_t>(), p.tp.perm.as<uint32_t>(), V, p.outdeg.as<uint32_t>());
-    OLV_TRY(p.contrib.ensure((size_t)V * 8 + 32));
+    k_outdeg_perm<<<g->num_sms * 8, kBlock, 0, g->stream>>>(g->rowptr.as<uint32_t>(), p.perm(), V,
+                                                           p.outdeg.as<uint32_t>());
+    OLV_TRY(p.contrib.ensure((size_t)V * 8 + 64));
     OLV_TRY(p.rank.ensure((size_t)V * 4 + 16));
     OLV_TRY(p.ctl.ensure(sizeof(PrCtl)));
     OLV_TRY(p.dang.ensure(16));
@@ -213,18 +285,16 @@ template <class Sink>
 static int pr_iteration(olv_graph *g, PrPlan &p, Sink &&sink, cudaGraphConditionalHandle h,
                         int use_cond) {
     PrCtl *ctl = p.ctl.as<PrCtl>();
-    PrOp op;
+    PrTileOp op;
     op.done = &ctl->done;
     op.ctl = ctl;
     op.c0 = p.contrib.as<float>();
     op.c1 = p.contrib.as<float>() + g->V;
     op.rank = p.rank.as<float>();
     op.outdeg = p.outdeg.as<uint32_t>();
-    op.a_hi = p.a_hi;
-    op.a_lo = p.a_lo;
     op.cin = nullptr;
     op.cout = nullptr;
-    op.base = 0;
+    op.a_hi = op.a_lo = op.base = 0;
     OLV_TRY(tile_pass(p.tp, op, sink));
     const double *cpart = p.tp.partials.as<double>();
     uint32_t nparts = kTileCTAs;
@@ -272,56 +342,82 @@ extern "C" int olv_pagerank(olv_graph *g, double alpha, int max_it, double tol, 
         }
     }
     PrPlan &p = ps->plan;
-    // alpha as an unevaluated FP32 pair so the update carries FP64-level alpha
     const double ad = alpha;
-    p.a_hi = (float)ad;
-    p.a_lo = (float)(ad - (double)p.a_hi);
     const bool dev_out = is_device_ptr(rank_out);
     if (!dev_out) OLV_TRY(g->ws.level.ensure((size_t)g->V * 4 + 16));
     float *rank = dev_out ? rank_out : g->ws.level.as<float>();
     float *rank_new = p.rank.as<float>();
 
+    const uint32_t leak = dangling_mode == OLV_DANGLING_LEAK ? 1u : 0u;
+    SolveCtl *sctl = p.sp.ctl.as<SolveCtl>();
     OLV_CUDA(cudaEventRecord(g->ev0, s));
-    OLV_CUDA(cudaMemsetAsync(p.dang.p, 0, 8, s));
-    k_pr_init<<<g->num_sms * 8, kBlock, 0, s>>>(p.outdeg.as<uint32_t>(), g->V, rank_new,
-                                               p.contrib.as<float>(),
-                                               p.dang.as<unsigned long long>());
-    k_pr_ctl_init<<<1, 1, 0, s>>>(p.ctl.as<PrCtl>(), p.dang.as<unsigned long long>(), g->V, ad,
-                                  (uint32_t)max_it, tol,
-                                  dangling_mode == OLV_DANGLING_LEAK ? 1u : 0u);
+    if (p.solve)
+        OLV_CUDA(cudaMemsetAsync(sctl, 0, sizeof(SolveCtl), s));
+    else
+        OLV_CUDA(cudaMemsetAsync(p.dang.p, 0, 8, s));
+    k_pr_init<<<g->num_sms * 8, kBlock, 0, s>>>(
+        p.outdeg.as<uint32_t>(), g->V, rank_new, p.contrib.as<float>(),
+        p.solve ? &sctl->count : p.dang.as<unsigned long long>());
     OLV_CUDA(cudaGetLastError());
-    bool launched = false;
-    if (g->tune.use_graphs && max_it > 0) {
-        if (!ps->graph.ready) {
-            int r = ps->graph.begin();
-            auto sink = [&](const void *f, dim3 gr, dim3 bl, void **args) {
-                return ps->graph.add(f, gr, bl, args);
+    if (p.solve) {
+        PrOp op = {};
+        op.c0 = p.contrib.as<float>();
+        op.c1 = op.c0 + (((size_t)g->V + 3) & ~(size_t)3);   // 16-byte aligned
+        op.rank = rank_new;
+        op.outdeg = p.outdeg.as<uint32_t>();
+        op.ctl = sctl;
+        op.alpha = ad;
+        op.a_hi = (float)ad;
+        op.a_lo = (float)(ad - (double)op.a_hi);
+        op.inv_n = 1.0 / (double)g->V;
+        op.leak = (int)leak;
+        op.rank0 = 1.0f / (float)g->V;
+        OLV_TRY(launch_solve(p.sp, p.sp.args((uint32_t)max_it, tol), op, s));
+    } else {
+        k_pr_ctl_init<<<1, 1, 0, s>>>(p.ctl.as<PrCtl>(), p.dang.as<unsigned long long>(), g->V, ad,
+                                      (uint32_t)max_it, tol, leak);
+        OLV_CUDA(cudaGetLastError());
+        bool launched = false;
+        if (g->tune.use_graphs && max_it > 0) {
+            if (!ps->graph.ready) {
+                int r = ps->graph.begin();
+                auto sink = [&](const void *f, dim3 gr, dim3 bl, void **args) {
+                    return ps->graph.add(f, gr, bl, args);
+                };
+                if (r == OLV_OK) r = pr_iteration(g, p, sink, ps->graph.handle, 1);
+                if (r == OLV_OK) r = ps->graph.finish();
+                if (r != OLV_OK) ps->graph.destroy();
+            }
+            if (ps->graph.ready) {
+                OLV_TRY(ps->graph.launch(s));
+                launched = true;
+            }
+        }
+        if (!launched) {
+            auto launch = [&](const void *f, dim3 gr, dim3 bl, void **args) {
+                OLV_CUDA(cudaLaunchKernel(f, gr, bl, args, 0, s));
+                return OLV_OK;
             };
-            if (r == OLV_OK) r = pr_iteration(g, p, sink, ps->graph.handle, 1);
-            if (r == OLV_OK) r = ps->graph.finish();
-            if (r != OLV_OK) ps->graph.destroy();
-        }
-        if (ps->graph.ready) {
-            OLV_TRY(ps->graph.launch(s));
-            launched = true;
+            for (int it = 0; it < max_it; it++) OLV_TRY(pr_iteration(g, p, launch, 0, 0));
         }
     }
-    if (!launched) {
-        auto launch = [&](const void *f, dim3 gr, dim3 bl, void **args) {
-            OLV_CUDA(cudaLaunchKernel(f, gr, bl, args, 0, s));
-            return OLV_OK;
-        };
-        for (int it = 0; it < max_it; it++) OLV_TRY(pr_iteration(g, p, launch, 0, 0));
-    }
-    k_pr_unpermute<<<g->num_sms * 8, kBlock, 0, s>>>(rank_new, p.tp.newid.as<uint32_t>(), g->V,
-                                                    rank);
+    k_pr_unpermute<<<g->num_sms * 8, kBlock, 0, s>>>(rank_new, p.newid(), g->V, rank);
     OLV_CUDA(cudaGetLastError());
     OLV_CUDA(cudaEventRecord(g->ev1, s));
-    PrCtl hc;
-    OLV_CUDA(cudaMemcpyAsync(&hc, p.ctl.p, sizeof(PrCtl), cudaMemcpyDeviceToHost, s));
+    PrCtl hc = {};
+    SolveCtl hs = {};
+    if (p.solve)
+        OLV_CUDA(cudaMemcpyAsync(&hs, sctl, sizeof hs, cudaMemcpyDeviceToHost, s));
+    else
+        OLV_CUDA(cudaMemcpyAsync(&hc, p.ctl.p, sizeof hc, cudaMemcpyDeviceToHost, s));
     if (!dev_out)
         OLV_CUDA(cudaMemcpyAsync(rank_out, rank, (size_t)g->V * 4, cudaMemcpyDeviceToHost, s));
     OLV_CUDA(cudaStreamSynchronize(s));
+    OLV_TRY(solve_error(hs, "olv_pagerank"));
+    if (p.solve) {
+        hc.iter = hs.iter;
+        hc.residual = hs.residual;
+    }
     if (st) {
         float ms = 0;
         OLV_CUDA(cudaEventElapsedTime(&ms, g->ev0, g->ev1));

@@ -61,19 +61,6 @@ struct PprCtl {
     uint32_t done;
 };
 
-// Two FP32 values in one 64-bit register and their lane-wise sums: sm_100a's
-// packed adds, each half rounded as a scalar add.
-__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b) {
-    unsigned long long d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-
 // Compensated accumulation of a lane's four vectors (Knuth's two-sum), two per
 // instruction: 14 instructions per in-edge and lane instead of 28 (the pass
 // was issue bound: 0.7 warp instructions per cycle and scheduler).

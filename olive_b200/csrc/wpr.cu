@@ -10,205 +10,258 @@
 // and FP64 residual norms, run as CUDA graphs; the gradient is implicit at the
 // fixed point, so memory is O(V + E) with no tape.
 //
-// The row sums run on row-reordered copies of the CSC (forward) and the CSR
-// (adjoint, W, t): rows sorted by length so that a group of 1..32 lanes per
-// row fits every row of a warp (olv_rowtiles.cuh); neighbour ids and all
-// per-vertex arrays keep the caller's numbering, and the edge weights are
-// permuted into each copy's entry order at the start of every forward solve.
-#include "olv_graphexec.cuh"
+// The row sums run on relabelled, row-sorted copies of the CSC (forward) and the
+// CSR (adjoint, W, t), a whole solve in one launch (olv_rowsolve.cuh); their
+// vectors are in each copy's numbering (hub values together, rows read and
+// written as runs) and the edge weights are permuted into each copy's entry
+// order at the start of every forward solve.  RMAT-20, 100 sweeps and their
+// adjoint: 20.2 -> 12.7 ms (before: rows reordered but ids and vectors in the
+// caller's numbering, L1 hits 21%, rows updated by scattered accesses).
 #include "olv_internal.cuh"
-#include "olv_rowtiles.cuh"
+#include "olv_rowsolve.cuh"
 
 struct olv_wpr_ctx {
     olv_graph *g = nullptr;
     double alpha = 0.85;
     float a_hi = 0, a_lo = 0;
-    olv::DevBuf W, r, s2, tp, lam2, t, gbuf;   // r: [V]; s2: 2V; lam2: 2V
-    olv::DevBuf ctl;                           // IterCtl
-    olv::WhileGraph fwd, bwd;
-    double fwd_alpha = -1, bwd_alpha = -1;
+    olv::DevBuf W, r, coef, lam, t, gbuf;      // [V], the caller's ids
+    olv::DevBuf fW, fr, ftp, fs2;              // forward (tcsc ids); fs2: ping-pong
+    olv::DevBuf aW, ag, alam2;                 // adjoint (tcsr ids); alam2: ping-pong
 };
 
 namespace olv {
 
 struct WprPlans {
-    RowPlan csr;               // row blocks of the CSR (gradient kernels)
-    TilePlan tcsc, tcsr;       // row-reordered CSC and CSR (row sums)
+    SolvePlan tcsc, tcsr;      // row-sorted CSC and CSR
     DevBuf wc, wr;             // weights in tcsc / tcsr entry order
+    DevBuf erow;               // gradient: row of every kGradEdges-th CSR entry
     ~WprPlans() {
-        csr.release();
         tcsc.release();
         tcsr.release();
         wc.release();
         wr.release();
+        erow.release();
     }
 };
 
-// --- row-sum ops ---------------------------------------------------------
-struct WsumOp {   // W_u = sum of out-weights (CSR)
-    const uint32_t *done;
-    const float *w;
+// --- row-sum ops (row ids are the plan's) ----------------------------------
+struct WsumOp {   // W_u = sum of out-weights (CSR), to the caller's ids
+    static constexpr bool kGather = false, kWeighted = true, kStore = false;
+    const uint32_t *perm;
     float *W;
-    __device__ __forceinline__ void begin() {}
-    __device__ __forceinline__ float term(uint32_t e, uint32_t) const { return __ldg(&w[e]); }
+    __device__ __forceinline__ double first_aux() const { return 0; }
+    __device__ __forceinline__ void begin(uint32_t, double) {}
+    __device__ __forceinline__ const float *in() const { return nullptr; }
+    __device__ __forceinline__ float *out() const { return nullptr; }
     struct Row {
-        uint32_t unused;
+        uint32_t v;
     };
-    __device__ __forceinline__ Row row(uint32_t) const { return Row{0}; }
-    __device__ __forceinline__ void finish(uint32_t u, float s, float c, const Row &, double &,
-                                           double &) const {
-        W[u] = s + c;
+    __device__ __forceinline__ Row row(uint32_t r) const { return Row{__ldg(&perm[r])}; }
+    __device__ __forceinline__ float finish(uint32_t, float s, float c, const Row &q, double &,
+                                            double &) const {
+        W[q.v] = s + c;
+        return 0.0f;
     }
 };
 
 struct WfwdOp {   // r'[v] = (1-alpha) p[v] + alpha sum_{u->v} w_uv r[u]/W_u
-    const uint32_t *done;
-    const IterCtl *ctl;
-    const float *wc;      // CSC-ordered weights
-    const float *s0, *s1; // r/W ping-pong
+    static constexpr bool kGather = true, kWeighted = true, kStore = true;
+    float *s0, *s1;       // r/W ping-pong
     const float *W, *tp;  // tp = (1-alpha) p
     float *r;
     float a_hi, a_lo;
-    const float *sin;
-    float *sout;
-    __device__ __forceinline__ void begin() {
-        const bool odd = ctl->iter & 1;
-        sin = odd ? s1 : s0;
-        sout = const_cast<float *>(odd ? s0 : s1);
-    }
-    __device__ __forceinline__ float term(uint32_t e, uint32_t u) const {
-        return __ldg(&wc[e]) * __ldg(&sin[u]);
-    }
+    uint32_t odd;
+    __device__ __forceinline__ double first_aux() const { return 0; }
+    __device__ __forceinline__ void begin(uint32_t it, double) { odd = it & 1; }
+    __device__ __forceinline__ const float *in() const { return odd ? s1 : s0; }
+    __device__ __forceinline__ float *out() const { return odd ? s0 : s1; }
     struct Row {
         float tp, r, W;
     };
-    __device__ __forceinline__ Row row(uint32_t v) const { return Row{tp[v], r[v], W[v]}; }
-    __device__ __forceinline__ void finish(uint32_t v, float s, float c, const Row &q, double &res,
-                                           double &) const {
+    __device__ __forceinline__ Row row(uint32_t v) const {
+        return Row{__ldg(&tp[v]), r[v], __ldg(&W[v])};
+    }
+    __device__ __forceinline__ float finish(uint32_t v, float s, float c, const Row &q, double &res,
+                                            double &) const {
         const float t = fmaf(a_lo, s, fmaf(a_hi, c, q.tp));
         const float nr = fmaf(a_hi, s, t);
         res += fabs((double)nr - (double)q.r);
         r[v] = nr;
-        sout[v] = q.W > 0.0f ? __fdiv_rn(nr, q.W) : 0.0f;
+        return q.W > 0.0f ? __fdiv_rn(nr, q.W) : 0.0f;
     }
 };
 
 struct WadjOp {   // lambda'[u] = g[u] + alpha sum_{u->v} w_uv lambda[v] / W_u
-    const uint32_t *done;
-    const IterCtl *ctl;
-    const float *w;        // CSR weights
-    const float *l0, *l1;  // lambda ping-pong
+    static constexpr bool kGather = true, kWeighted = true, kStore = true;
+    float *l0, *l1;        // lambda ping-pong
     const float *W, *gv;
-    float *t;              // t_u of the sweep (for the gradient)
     float a_hi, a_lo;
-    const float *lin;
-    float *lout;
-    __device__ __forceinline__ void begin() {
-        const bool odd = ctl->iter & 1;
-        lin = odd ? l1 : l0;
-        lout = const_cast<float *>(odd ? l0 : l1);
-    }
-    __device__ __forceinline__ float term(uint32_t e, uint32_t v) const {
-        return __ldg(&w[e]) * __ldg(&lin[v]);
-    }
+    uint32_t odd;
+    __device__ __forceinline__ double first_aux() const { return 0; }
+    __device__ __forceinline__ void begin(uint32_t it, double) { odd = it & 1; }
+    __device__ __forceinline__ const float *in() const { return odd ? l1 : l0; }
+    __device__ __forceinline__ float *out() const { return odd ? l0 : l1; }
     struct Row {
         float W, g, lam;
     };
-    __device__ __forceinline__ Row row(uint32_t u) const { return Row{W[u], gv[u], lin[u]}; }
-    __device__ __forceinline__ void finish(uint32_t u, float s, float c, const Row &q, double &res,
-                                           double &) const {
+    __device__ __forceinline__ Row row(uint32_t u) const {
+        return Row{__ldg(&W[u]), __ldg(&gv[u]), __ldcg(&in()[u])};
+    }
+    __device__ __forceinline__ float finish(uint32_t, float s, float c, const Row &q, double &res,
+                                            double &) const {
         const float tu = q.W > 0.0f ? __fdiv_rn(s + c, q.W) : 0.0f;
         const float nl = fmaf(a_hi, tu, fmaf(a_lo, tu, q.g));
         res += fabs((double)nl - (double)q.lam);
-        lout[u] = nl;
-        t[u] = tu;
+        return nl;
     }
 };
 
-struct WtOp {     // t_u from the final lambda, and dL/dp = (1-alpha) lambda
-    const uint32_t *done;
-    const float *w, *lam, *W;
-    float *t, *dp;
-    float one_minus_alpha;
-    __device__ __forceinline__ void begin() {}
-    __device__ __forceinline__ float term(uint32_t e, uint32_t v) const {
-        return __ldg(&w[e]) * __ldg(&lam[v]);
-    }
+// One pass over the final lambda: t_u, lambda, dL/dp = (1-alpha) lambda and the
+// gradient's row factor alpha r_u / W_u, all in the caller's ids.
+struct WtOp {
+    static constexpr bool kGather = true, kWeighted = true, kStore = false;
+    const float *l0, *l1;
+    const uint32_t *sweeps;   // adjoint sweeps run: which buffer holds lambda
+    const uint32_t *perm;
+    const float *W, *r;       // W in row ids, r in the caller's
+    float *t, *lam, *coef, *dp;
+    float alpha, one_minus_alpha;
+    const float *l;
+    __device__ __forceinline__ double first_aux() const { return 0; }
+    __device__ __forceinline__ void begin(uint32_t, double) { l = (*sweeps & 1) ? l1 : l0; }
+    __device__ __forceinline__ const float *in() const { return l; }
+    __device__ __forceinline__ float *out() const { return nullptr; }
     struct Row {
-        float W, lam;
+        float W, lam, r;
+        uint32_t v;
     };
-    __device__ __forceinline__ Row row(uint32_t u) const { return Row{W[u], lam[u]}; }
-    __device__ __forceinline__ void finish(uint32_t u, float s, float c, const Row &q, double &,
-                                           double &) const {
-        t[u] = q.W > 0.0f ? __fdiv_rn(s + c, q.W) : 0.0f;
-        if (dp) dp[u] = one_minus_alpha * q.lam;
+    __device__ __forceinline__ Row row(uint32_t u) const {
+        const uint32_t v = __ldg(&perm[u]);
+        return Row{__ldg(&W[u]), __ldg(&l[u]), __ldg(&r[v]), v};
+    }
+    __device__ __forceinline__ float finish(uint32_t, float s, float c, const Row &q, double &,
+                                            double &) const {
+        t[q.v] = q.W > 0.0f ? __fdiv_rn(s + c, q.W) : 0.0f;
+        lam[q.v] = q.lam;
+        coef[q.v] = q.W > 0.0f ? __fdiv_rn(alpha * q.r, q.W) : 0.0f;
+        if (dp) dp[q.v] = one_minus_alpha * q.lam;
+        return 0.0f;
     }
 };
 
-// dL/dw_e for the CSR edges of a row block (rows found by binary search in
-// shared memory), or of one long-row segment.
-__global__ void __launch_bounds__(kBlock)
-k_wpr_grad_blocks(const uint32_t *__restrict__ ptr, const uint32_t *__restrict__ col,
-                  const uint32_t *__restrict__ blocks, const float *__restrict__ r,
-                  const float *__restrict__ W, const float *__restrict__ lam,
-                  const float *__restrict__ t, float alpha, float *__restrict__ dw) {
-    const uint32_t r0 = blocks[blockIdx.x], r1 = blocks[blockIdx.x + 1];
-    const uint32_t e0 = ptr[r0], e1 = ptr[r1];
-    if (e1 - e0 > kNnz) return;   // long rows: k_wpr_grad_segments
-    __shared__ uint32_t s_ptr[kRows + 1];
-    const uint32_t nr = r1 - r0;
-    for (uint32_t i = threadIdx.x; i <= nr; i += kBlock) s_ptr[i] = ptr[r0 + i];
-    __syncthreads();
-    for (uint32_t e = e0 + threadIdx.x; e < e1; e += kBlock) {
-        uint32_t lo = 0, hi = nr;   // largest k with s_ptr[k] <= e
-        while (hi - lo > 1) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (s_ptr[mid] <= e) lo = mid; else hi = mid;
-        }
-        const uint32_t u = r0 + lo;
-        const float Wu = W[u];
-        const float coef = Wu > 0.0f ? __fdiv_rn(alpha * r[u], Wu) : 0.0f;
-        dw[e] = coef * (__ldg(&lam[col[e]]) - t[u]);
+// Row of CSR entry e: the last one that begins at or before e.
+__device__ __forceinline__ uint32_t row_of(const uint32_t *__restrict__ ptr, uint32_t V,
+                                           uint64_t e) {
+    uint32_t lo = 0, hi = V;   // ptr[lo] <= e < ptr[hi]
+    while (hi - lo > 1) {
+        const uint32_t mid = lo + (hi - lo) / 2;
+        if (__ldg(&ptr[mid]) <= e)
+            lo = mid;
+        else
+            hi = mid;
     }
+    return lo;
 }
 
-__global__ void __launch_bounds__(kBlock)
-k_wpr_grad_segments(const uint32_t *__restrict__ col, const uint2 *__restrict__ seg_range,
-                    const uint32_t *__restrict__ seg_row, const float *__restrict__ r,
-                    const float *__restrict__ W, const float *__restrict__ lam,
-                    const float *__restrict__ t, float alpha, float *__restrict__ dw) {
-    const uint2 sr = seg_range[blockIdx.x];
-    const uint32_t u = seg_row[blockIdx.x];
-    const float Wu = W[u];
-    const float coef = Wu > 0.0f ? __fdiv_rn(alpha * r[u], Wu) : 0.0f;
-    const float tu = t[u];
-    for (uint32_t e = sr.x + threadIdx.x; e < sr.y; e += kBlock)
-        dw[e] = coef * (__ldg(&lam[col[e]]) - tu);
-}
+constexpr uint32_t kGradEdges = 256;   // entries a warp takes at a time
 
-__global__ void k_wpr_init(uint32_t V, const float *p, const float *W, float alpha, float *tp,
-                           float *r, float *s0) {
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V;
-         v += (uint64_t)gridDim.x * blockDim.x) {
-        const float pv = p[v];
-        tp[v] = (1.0f - alpha) * pv;
-        r[v] = pv;
-        s0[v] = W[v] > 0.0f ? __fdiv_rn(pv, W[v]) : 0.0f;
-    }
-}
-
-__global__ void k_copy_f32(const float *__restrict__ a, float *__restrict__ b, uint32_t n) {
+__global__ void k_grad_rows(const uint32_t *__restrict__ ptr, uint32_t V, uint64_t E,
+                            uint32_t *__restrict__ erow) {
+    const uint64_t n = (E + kGradEdges - 1) / kGradEdges;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
          i += (uint64_t)gridDim.x * blockDim.x)
-        b[i] = a[i];
+        erow[i] = row_of(ptr, V, i * kGradEdges);
 }
 
-__global__ void k_iter_init(IterCtl *c, uint32_t max_it, double tol) {
-    IterCtl t = {};
-    t.max_it = max_it;
-    t.tol = tol;
-    t.done = max_it == 0;
-    *c = t;
+// dL/dw_e = coef[u] (lambda[col e] - t[u]), u the row of entry e.  A warp takes
+// kGradEdges entries from a known first row; a lane's rows only go up, so each
+// entry's row is found by stepping on from the last one's, or by a search in the
+// rows left when they are many.
+__global__ void __launch_bounds__(kBlock)
+k_wpr_grad(const uint32_t *__restrict__ ptr, const uint32_t *__restrict__ col, uint32_t V,
+           uint64_t E, const uint32_t *__restrict__ erow, const float *__restrict__ coef,
+           const float *__restrict__ lam, const float *__restrict__ t, float *__restrict__ dw) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t n = (E + kGradEdges - 1) / kGradEdges;
+    const uint64_t warp = (blockIdx.x * (uint64_t)kBlock + threadIdx.x) >> 5;
+    const uint64_t nwarps = ((uint64_t)gridDim.x * kBlock) >> 5;
+    for (uint64_t i = warp; i < n; i += nwarps) {
+        const uint32_t r0 = __ldg(&erow[i]), r1 = i + 1 < n ? __ldg(&erow[i + 1]) : V - 1;
+        constexpr int kSteps = kGradEdges / 32;
+        uint32_t c[kSteps], u[kSteps];
+        float l[kSteps];
+#pragma unroll
+        for (int q = 0; q < kSteps; q++) {
+            const uint64_t e = i * kGradEdges + q * 32 + lane;
+            c[q] = e < E ? __ldg(&col[e]) : 0u;
+        }
+#pragma unroll
+        for (int q = 0; q < kSteps; q++) l[q] = __ldg(&lam[c[q]]);
+        uint32_t lo = r0;
+#pragma unroll
+        for (int q = 0; q < kSteps; q++) {
+            const uint64_t e = i * kGradEdges + q * 32 + lane;
+            uint32_t hi = r1 + 1;
+            while (hi - lo > 1) {   // the row lies in [lo, hi)
+                const uint32_t mid = lo + (hi - lo) / 2;
+                if (__ldg(&ptr[mid]) <= e)
+                    lo = mid;
+                else
+                    hi = mid;
+            }
+            u[q] = lo;
+        }
+#pragma unroll
+        for (int q = 0; q < kSteps; q++) {
+            const uint64_t e = i * kGradEdges + q * 32 + lane;
+            if (e < E) dw[e] = __ldg(&coef[u[q]]) * (l[q] - __ldg(&t[u[q]]));
+        }
+    }
+}
+
+// Weights in a plan's entry order; places without an entry weigh nothing.
+__global__ void k_permute_entries(const float *__restrict__ in, const uint32_t *__restrict__ pos,
+                                  uint64_t n, float *__restrict__ out) {
+    for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < n;
+         k += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t p = pos[k];
+        out[k] = p != 0xffffffffu ? in[p] : 0.0f;
+    }
+}
+
+// Start of a forward solve, in the plan's ids.
+__global__ void k_wpr_init(uint32_t V, const float *__restrict__ p, const float *__restrict__ W,
+                           const uint32_t *__restrict__ perm, float alpha, float *tp, float *r,
+                           float *s0, float *Wp) {
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < V;
+         i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t v = perm[i];
+        const float pv = p[v], wv = W[v];
+        tp[i] = (1.0f - alpha) * pv;
+        r[i] = pv;
+        Wp[i] = wv;
+        s0[i] = wv > 0.0f ? __fdiv_rn(pv, wv) : 0.0f;
+    }
+}
+
+// Start of an adjoint solve, in the plan's ids.
+__global__ void k_wadj_init(uint32_t V, const float *__restrict__ g, const float *__restrict__ W,
+                            const uint32_t *__restrict__ perm, float *gp, float *l0, float *Wp) {
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < V;
+         i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t v = perm[i];
+        gp[i] = g[v];
+        l0[i] = g[v];
+        Wp[i] = W[v];
+    }
+}
+
+// out[v] = in[newid[v]]
+__global__ void k_to_ids(const float *__restrict__ in, const uint32_t *__restrict__ newid,
+                         uint32_t V, float *__restrict__ out) {
+    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V;
+         v += (uint64_t)gridDim.x * blockDim.x)
+        out[v] = in[newid[v]];
 }
 
 static WprPlans *wpr_plans(olv_graph *g) { return static_cast<WprPlans *>(g->wpr_state); }
@@ -216,19 +269,22 @@ static WprPlans *wpr_plans(olv_graph *g) { return static_cast<WprPlans *>(g->wpr
 static int ensure_wpr_plans(olv_graph *g) {
     if (g->wpr_state) return OLV_OK;
     WprPlans *p = new WprPlans();
-    int r = build_row_plan(g->rowptr.as<uint32_t>(), g->V, g->stream, p->csr);
+    cudaStream_t s = g->stream;
+    int r = build_solve_plan(g->colptr.as<uint32_t>(), g->rowidx.as<uint32_t>(),
+                             g->csc_eid.as<uint32_t>(), g->V, g->E, g->tune.pr_tile_u, true,
+                             g->num_sms, s, p->tcsc);
     if (r == OLV_OK)
-        r = build_tile_plan(g->colptr.as<uint32_t>(), g->rowidx.as<uint32_t>(), g->V, g->stream,
-                            p->tcsc, false, g->tune.pr_tile_u);
-    if (r == OLV_OK)
-        r = build_tile_plan(g->rowptr.as<uint32_t>(), g->col.as<uint32_t>(), g->V, g->stream,
-                            p->tcsr, false, g->tune.pr_tile_u);
-    if (r == OLV_OK) r = p->wc.ensure(g->E * 4 + 16);
-    if (r == OLV_OK) r = p->wr.ensure(g->E * 4 + 16);
+        r = build_solve_plan(g->rowptr.as<uint32_t>(), g->col.as<uint32_t>(), nullptr, g->V, g->E,
+                             g->tune.pr_tile_u, true, g->num_sms, s, p->tcsr);
+    if (r == OLV_OK) r = p->wc.ensure(p->tcsc.entries * 4 + 16);
+    if (r == OLV_OK) r = p->wr.ensure(p->tcsr.entries * 4 + 16);
+    if (r == OLV_OK) r = p->erow.ensure((g->E / kGradEdges + 1) * 4);
     if (r != OLV_OK) {
         delete p;
         return r;
     }
+    k_grad_rows<<<g->num_sms * 8, kBlock, 0, s>>>(g->rowptr.as<uint32_t>(), g->V, g->E,
+                                                 p->erow.as<uint32_t>());
     g->wpr_state = p;
     return OLV_OK;
 }
@@ -277,89 +333,48 @@ extern "C" int olv_wpr_forward(olv_graph *g, const float *w, const float *p, dou
     split_alpha(alpha, c->a_hi, c->a_lo);
     const size_t V = g->V;
     cudaStream_t s = g->stream;
-    OLV_TRY(c->W.ensure(V * 4 + 16));
-    OLV_TRY(c->r.ensure(V * 4 + 16));
-    OLV_TRY(c->s2.ensure(V * 8 + 32));
-    OLV_TRY(c->tp.ensure(V * 4 + 16));
-    OLV_TRY(c->ctl.ensure(sizeof(IterCtl)));
+    const size_t Va = (V + 3) & ~(size_t)3;   // ping-pong halves 16-byte aligned
+    for (DevBuf *b : {&c->W, &c->r, &c->fW, &c->fr, &c->ftp}) OLV_TRY(b->ensure(V * 4 + 16));
+    OLV_TRY(c->fs2.ensure(Va * 8 + 32));
     OLV_TRY(copy_vec_in(c->gbuf, p, V, s));   // p staged in gbuf during the forward
-    IterCtl *ctl = c->ctl.as<IterCtl>();
+    SolveCtl *fctl = pl.tcsc.ctl.as<SolveCtl>(), *rctl = pl.tcsr.ctl.as<SolveCtl>();
     OLV_CUDA(cudaEventRecord(g->ev0, s));
-    // the weights in the entry orders of the two row-reordered copies
-    k_permute_entries<<<g->num_sms * 8, kBlock, 0, s>>>(g->csc_w.as<float>(),
-                                                       pl.tcsc.pos.as<uint32_t>(), g->E,
+    OLV_CUDA(cudaMemsetAsync(fctl, 0, sizeof(SolveCtl), s));
+    OLV_CUDA(cudaMemsetAsync(rctl, 0, sizeof(SolveCtl), s));
+    // the weights in the entry orders of the two copies
+    k_permute_entries<<<g->num_sms * 8, kBlock, 0, s>>>(g->w.as<float>(),
+                                                       pl.tcsc.pos.as<uint32_t>(), pl.tcsc.entries,
                                                        pl.wc.as<float>());
     k_permute_entries<<<g->num_sms * 8, kBlock, 0, s>>>(g->w.as<float>(),
-                                                       pl.tcsr.pos.as<uint32_t>(), g->E,
+                                                       pl.tcsr.pos.as<uint32_t>(), pl.tcsr.entries,
                                                        pl.wr.as<float>());
     // W = row sums of the weights (one pass, same deterministic engine)
-    {
-        k_iter_init<<<1, 1, 0, s>>>(ctl, 1, 0.0);   // done = 0 for the single pass
-        PermOp<WsumOp> op{WsumOp{&ctl->done, pl.wr.as<float>(), c->W.as<float>()},
-                          pl.tcsr.perm.as<uint32_t>(), &ctl->done};
-        auto launch = [&](const void *f, dim3 gr, dim3 bl, void **args) {
-            OLV_CUDA(cudaLaunchKernel(f, gr, bl, args, 0, s));
-            return OLV_OK;
-        };
-        OLV_TRY(tile_pass(pl.tcsr, op, launch));
-    }
-    k_wpr_init<<<g->num_sms * 8, kBlock, 0, s>>>(g->V, c->gbuf.as<float>(), c->W.as<float>(),
-                                                (float)alpha, c->tp.as<float>(), c->r.as<float>(),
-                                                c->s2.as<float>());
-    k_iter_init<<<1, 1, 0, s>>>(ctl, (uint32_t)max_it, tol);
+    OLV_TRY(launch_solve(pl.tcsr, pl.tcsr.args(1, 0.0, &pl.wr),
+                         WsumOp{pl.tcsr.perm.as<uint32_t>(), c->W.as<float>()}, s));
+    k_wpr_init<<<g->num_sms * 8, kBlock, 0, s>>>(
+        g->V, c->gbuf.as<float>(), c->W.as<float>(), pl.tcsc.perm.as<uint32_t>(), (float)alpha,
+        c->ftp.as<float>(), c->fr.as<float>(), c->fs2.as<float>(), c->fW.as<float>());
     OLV_CUDA(cudaGetLastError());
-    WfwdOp fop;
-    WfwdOp &op = fop;
-    op.done = &ctl->done;
-    op.ctl = ctl;
-    op.wc = pl.wc.as<float>();
-    op.s0 = c->s2.as<float>();
-    op.s1 = c->s2.as<float>() + V;
-    op.W = c->W.as<float>();
-    op.tp = c->tp.as<float>();
-    op.r = c->r.as<float>();
+    WfwdOp op = {};
+    op.s0 = c->fs2.as<float>();
+    op.s1 = op.s0 + Va;
+    op.W = c->fW.as<float>();
+    op.tp = c->ftp.as<float>();
+    op.r = c->fr.as<float>();
     op.a_hi = c->a_hi;
     op.a_lo = c->a_lo;
-    op.sin = nullptr;
-    op.sout = nullptr;
-    PermOp<WfwdOp> pop{fop, pl.tcsc.perm.as<uint32_t>(), &ctl->done};
-    const double *cpart = pl.tcsc.partials.as<double>();
-    uint32_t nparts = kTileCTAs;
-    auto body = [&](auto &&sink, cudaGraphConditionalHandle h, int use_cond) {
-        OLV_TRY(tile_pass(pl.tcsc, pop, sink));
-        void *a_fold[] = {&ctl, &cpart, &nparts, &h, &use_cond};
-        return sink((const void *)k_iter_fold, dim3(1), dim3(kFoldThreads), a_fold);
-    };
-    bool launched = false;
-    if (c->fwd.ready && c->fwd_alpha != alpha) c->fwd.destroy();
-    if (g->tune.use_graphs && max_it > 0) {
-        if (!c->fwd.ready) {
-            c->fwd_alpha = alpha;
-            int r = c->fwd.begin();
-            auto sink = [&](const void *f, dim3 gr, dim3 bl, void **args) {
-                return c->fwd.add(f, gr, bl, args);
-            };
-            if (r == OLV_OK) r = body(sink, c->fwd.handle, 1);
-            if (r == OLV_OK) r = c->fwd.finish();
-            if (r != OLV_OK) c->fwd.destroy();
-        }
-        if (c->fwd.ready) {
-            OLV_TRY(c->fwd.launch(s));
-            launched = true;
-        }
-    }
-    if (!launched) {
-        auto launch = [&](const void *f, dim3 gr, dim3 bl, void **args) {
-            OLV_CUDA(cudaLaunchKernel(f, gr, bl, args, 0, s));
-            return OLV_OK;
-        };
-        for (int i = 0; i < max_it; i++) OLV_TRY(body(launch, 0, 0));
-    }
+    OLV_TRY(launch_solve(pl.tcsc, pl.tcsc.args((uint32_t)max_it, tol, &pl.wc), op, s));
+    k_to_ids<<<g->num_sms * 8, kBlock, 0, s>>>(c->fr.as<float>(), pl.tcsc.newid.as<uint32_t>(),
+                                              g->V, c->r.as<float>());
+    OLV_CUDA(cudaGetLastError());
     OLV_CUDA(cudaEventRecord(g->ev1, s));
-    IterCtl hc;
-    OLV_CUDA(cudaMemcpyAsync(&hc, ctl, sizeof hc, cudaMemcpyDeviceToHost, s));
+    SolveCtl hc, hr;
+    OLV_CUDA(cudaMemcpyAsync(&hc, fctl, sizeof hc, cudaMemcpyDeviceToHost, s));
+    OLV_CUDA(cudaMemcpyAsync(&hr, rctl, sizeof hr, cudaMemcpyDeviceToHost, s));
     if (r_out) OLV_CUDA(cudaMemcpyAsync(r_out, c->r.p, V * 4, cudaMemcpyDefault, s));
     OLV_CUDA(cudaStreamSynchronize(s));
+    OLV_TRY(solve_error(hc, "olv_wpr_forward"));
+    OLV_TRY(solve_error(hr, "olv_wpr_forward"));
     if (st) {
         float ms = 0;
         OLV_CUDA(cudaEventElapsedTime(&ms, g->ev0, g->ev1));
@@ -388,8 +403,9 @@ extern "C" int olv_wpr_backward(olv_wpr_ctx *c, const float *gvec, int max_it, d
     const size_t V = g->V;
     const uint64_t E = g->E;
     cudaStream_t s = g->stream;
-    OLV_TRY(c->lam2.ensure(V * 8 + 32));
-    OLV_TRY(c->t.ensure(V * 4 + 16));
+    const size_t Va = (V + 3) & ~(size_t)3;
+    for (DevBuf *b : {&c->coef, &c->lam, &c->t, &c->aW, &c->ag}) OLV_TRY(b->ensure(V * 4 + 16));
+    OLV_TRY(c->alam2.ensure(Va * 8 + 32));
     OLV_TRY(copy_vec_in(c->gbuf, gvec, V, s));
     const bool dev_dw = is_device_ptr(dw_out);
     const bool dev_dp = dp_out && is_device_ptr(dp_out);
@@ -398,86 +414,54 @@ extern "C" int olv_wpr_backward(olv_wpr_ctx *c, const float *gvec, int max_it, d
     if (dp_out && !dev_dp) OLV_TRY(dpbuf.ensure(V * 4 + 16));
     float *dw = dev_dw ? dw_out : dwbuf.as<float>();
     float *dp = dp_out ? (dev_dp ? dp_out : dpbuf.as<float>()) : nullptr;
-    IterCtl *ctl = c->ctl.as<IterCtl>();
+    SolveCtl *ctl = pl.tcsr.ctl.as<SolveCtl>();
     OLV_CUDA(cudaEventRecord(g->ev0, s));
-    k_copy_f32<<<g->num_sms * 8, kBlock, 0, s>>>(c->gbuf.as<float>(), c->lam2.as<float>(), g->V);
-    k_iter_init<<<1, 1, 0, s>>>(ctl, (uint32_t)max_it, tol);
+    OLV_CUDA(cudaMemsetAsync(ctl, 0, sizeof(SolveCtl), s));
+    k_wadj_init<<<g->num_sms * 8, kBlock, 0, s>>>(
+        g->V, c->gbuf.as<float>(), c->W.as<float>(), pl.tcsr.perm.as<uint32_t>(),
+        c->ag.as<float>(), c->alam2.as<float>(), c->aW.as<float>());
     OLV_CUDA(cudaGetLastError());
-    WadjOp aop;
-    WadjOp &op = aop;
-    op.done = &ctl->done;
-    op.ctl = ctl;
-    op.w = pl.wr.as<float>();
-    op.l0 = c->lam2.as<float>();
-    op.l1 = c->lam2.as<float>() + V;
-    op.W = c->W.as<float>();
-    op.gv = c->gbuf.as<float>();
-    op.t = c->t.as<float>();
+    WadjOp op = {};
+    op.l0 = c->alam2.as<float>();
+    op.l1 = op.l0 + Va;
+    op.W = c->aW.as<float>();
+    op.gv = c->ag.as<float>();
     op.a_hi = c->a_hi;
     op.a_lo = c->a_lo;
-    op.lin = nullptr;
-    op.lout = nullptr;
-    PermOp<WadjOp> pop{aop, pl.tcsr.perm.as<uint32_t>(), &ctl->done};
-    const double *cpart = pl.tcsr.partials.as<double>();
-    uint32_t nparts = kTileCTAs;
-    auto body = [&](auto &&sink, cudaGraphConditionalHandle h, int use_cond) {
-        OLV_TRY(tile_pass(pl.tcsr, pop, sink));
-        void *a_fold[] = {&ctl, &cpart, &nparts, &h, &use_cond};
-        return sink((const void *)k_iter_fold, dim3(1), dim3(kFoldThreads), a_fold);
-    };
-    bool launched = false;
-    if (c->bwd.ready && c->bwd_alpha != c->alpha) c->bwd.destroy();
-    if (g->tune.use_graphs && max_it > 0) {
-        if (!c->bwd.ready) {
-            c->bwd_alpha = c->alpha;
-            int r = c->bwd.begin();
-            auto sink = [&](const void *f, dim3 gr, dim3 bl, void **args) {
-                return c->bwd.add(f, gr, bl, args);
-            };
-            if (r == OLV_OK) r = body(sink, c->bwd.handle, 1);
-            if (r == OLV_OK) r = c->bwd.finish();
-            if (r != OLV_OK) c->bwd.destroy();
-        }
-        if (c->bwd.ready) {
-            OLV_TRY(c->bwd.launch(s));
-            launched = true;
-        }
-    }
-    if (!launched) {
-        auto launch = [&](const void *f, dim3 gr, dim3 bl, void **args) {
-            OLV_CUDA(cudaLaunchKernel(f, gr, bl, args, 0, s));
-            return OLV_OK;
-        };
-        for (int i = 0; i < max_it; i++) OLV_TRY(body(launch, 0, 0));
-    }
-    IterCtl hc;
+    OLV_TRY(launch_solve(pl.tcsr, pl.tcsr.args((uint32_t)max_it, tol, &pl.wr), op, s));
+    SolveCtl hc, ht;
     OLV_CUDA(cudaMemcpyAsync(&hc, ctl, sizeof hc, cudaMemcpyDeviceToHost, s));
-    OLV_CUDA(cudaStreamSynchronize(s));
-    // final lambda lives in the buffer the last sweep wrote
-    const float *lam = c->lam2.as<float>() + ((hc.iter & 1) ? V : 0);
-    {
-        k_iter_init<<<1, 1, 0, s>>>(ctl, 1, 0.0);
-        PermOp<WtOp> top{WtOp{&ctl->done, pl.wr.as<float>(), lam, c->W.as<float>(),
-                              c->t.as<float>(), dp, (float)(1.0 - c->alpha)},
-                         pl.tcsr.perm.as<uint32_t>(), &ctl->done};
-        auto launch = [&](const void *f, dim3 gr, dim3 bl, void **args) {
-            OLV_CUDA(cudaLaunchKernel(f, gr, bl, args, 0, s));
-            return OLV_OK;
-        };
-        OLV_TRY(tile_pass(pl.tcsr, top, launch));
-    }
-    k_wpr_grad_blocks<<<pl.csr.nblocks, kBlock, 0, s>>>(
-        g->rowptr.as<uint32_t>(), g->col.as<uint32_t>(), pl.csr.blocks.as<uint32_t>(),
-        c->r.as<float>(), c->W.as<float>(), lam, c->t.as<float>(), (float)c->alpha, dw);
-    if (pl.csr.nsegs)
-        k_wpr_grad_segments<<<pl.csr.nsegs, kBlock, 0, s>>>(
-            g->col.as<uint32_t>(), pl.csr.seg_range.as<uint2>(), pl.csr.seg_row.as<uint32_t>(),
-            c->r.as<float>(), c->W.as<float>(), lam, c->t.as<float>(), (float)c->alpha, dw);
+    // the last pass counts its own barrier and iteration in tcsc's block
+    SolveCtl *tctl = pl.tcsc.ctl.as<SolveCtl>();
+    OLV_CUDA(cudaMemsetAsync(tctl, 0, sizeof(SolveCtl), s));
+    WtOp top = {};
+    top.l0 = op.l0;
+    top.l1 = op.l1;
+    top.sweeps = &ctl->iter;
+    top.perm = pl.tcsr.perm.as<uint32_t>();
+    top.W = c->aW.as<float>();
+    top.r = c->r.as<float>();
+    top.t = c->t.as<float>();
+    top.lam = c->lam.as<float>();
+    top.coef = c->coef.as<float>();
+    top.dp = dp;
+    top.alpha = (float)c->alpha;
+    top.one_minus_alpha = (float)(1.0 - c->alpha);
+    SolveArgs ta = pl.tcsr.args(1, 0.0, &pl.wr);
+    ta.ctl = tctl;
+    OLV_TRY(launch_solve(pl.tcsr, ta, top, s));
+    OLV_CUDA(cudaMemcpyAsync(&ht, tctl, sizeof ht, cudaMemcpyDeviceToHost, s));
+    if (E)
+        k_wpr_grad<<<g->num_sms * 8, kBlock, 0, s>>>(
+            g->rowptr.as<uint32_t>(), g->col.as<uint32_t>(), g->V, E, pl.erow.as<uint32_t>(),
+            c->coef.as<float>(), c->lam.as<float>(), c->t.as<float>(), dw);
     OLV_CUDA(cudaGetLastError());
     OLV_CUDA(cudaEventRecord(g->ev1, s));
     if (!dev_dw) OLV_CUDA(cudaMemcpyAsync(dw_out, dw, E * 4, cudaMemcpyDeviceToHost, s));
     if (dp_out && !dev_dp) OLV_CUDA(cudaMemcpyAsync(dp_out, dp, V * 4, cudaMemcpyDeviceToHost, s));
     OLV_CUDA(cudaStreamSynchronize(s));
+    OLV_TRY(solve_error(hc, "olv_wpr_backward"));
+    OLV_TRY(solve_error(ht, "olv_wpr_backward"));
     if (st) {
         float ms = 0;
         OLV_CUDA(cudaEventElapsedTime(&ms, g->ev0, g->ev1));
@@ -494,10 +478,6 @@ extern "C" int olv_wpr_backward(olv_wpr_ctx *c, const float *gvec, int max_it, d
 
 extern "C" int olv_wpr_ctx_destroy(olv_wpr_ctx *c) {
     if (!c) return OLV_OK;
-    c->fwd.destroy();
-    c->bwd.destroy();
-    c->W.release(); c->r.release(); c->s2.release(); c->tp.release(); c->lam2.release();
-    c->t.release(); c->gbuf.release(); c->ctl.release();
     delete c;
     return OLV_OK;
 }
