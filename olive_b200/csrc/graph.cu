@@ -267,6 +267,55 @@ static int copy_in(DevBuf &dst, const void *src, size_t bytes, cudaStream_t s) {
     return OLV_OK;
 }
 
+// The caller's CSR, checked where it now is: rowptr[0] == 0, rowptr[V] == E, rows
+// non-decreasing, every column below V.  bad[0], bad[1]: the first decreasing row
+// and the first column out of range.  (On the host the copy back and the loop
+// took longer than everything else in a graph of 16 M edges.)
+__global__ void k_check_csr(const uint32_t *__restrict__ rowptr, const uint32_t *__restrict__ col,
+                            uint32_t V, uint64_t E, unsigned long long *__restrict__ bad) {
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    unsigned long long row = ~0ULL, c = ~0ULL;
+    for (uint64_t v = tid; v < V; v += stride)
+        if (rowptr[v + 1] < rowptr[v] && row == ~0ULL) row = v;
+    for (uint64_t i = tid; i < E; i += stride)
+        if (col[i] >= V && c == ~0ULL) c = i;
+    if (row != ~0ULL) atomicMin(&bad[0], row);
+    if (c != ~0ULL) atomicMin(&bad[1], c);
+}
+
+static int check_csr(olv_graph *g) {
+    cudaStream_t s = g->stream;
+    DevBuf bad;
+    OLV_TRY(bad.ensure(16));
+    OLV_CUDA(cudaMemsetAsync(bad.p, 0xff, 16, s));
+    k_check_csr<<<grid_for(g->E + g->V, g->num_sms), kBlock, 0, s>>>(
+        g->rowptr.as<uint32_t>(), g->col.as<uint32_t>(), g->V, g->E, bad.as<unsigned long long>());
+    unsigned long long h[2];
+    uint32_t ends[2];
+    OLV_CUDA(cudaGetLastError());
+    OLV_CUDA(cudaMemcpyAsync(h, bad.p, 16, cudaMemcpyDeviceToHost, s));
+    OLV_CUDA(cudaMemcpyAsync(&ends[0], g->rowptr.p, 4, cudaMemcpyDeviceToHost, s));
+    OLV_CUDA(cudaMemcpyAsync(&ends[1], g->rowptr.as<uint32_t>() + g->V, 4, cudaMemcpyDeviceToHost, s));
+    OLV_CUDA(cudaStreamSynchronize(s));
+    if (ends[0] != 0 || ends[1] != g->E) {
+        set_error("olv_graph_create: rowptr[0]=%u rowptr[V]=%u, expected 0 and E=%llu", ends[0],
+                  ends[1], (unsigned long long)g->E);
+        return OLV_ERR_ARG;
+    }
+    if (h[0] != ~0ULL) {
+        set_error("olv_graph_create: rowptr decreases at vertex %llu", h[0]);
+        return OLV_ERR_ARG;
+    }
+    if (h[1] != ~0ULL) {
+        uint32_t c = 0;
+        OLV_CUDA(cudaMemcpy(&c, g->col.as<uint32_t>() + h[1], 4, cudaMemcpyDeviceToHost));
+        set_error("olv_graph_create: col[%llu]=%u out of range (V=%u)", h[1], c, g->V);
+        return OLV_ERR_ARG;
+    }
+    return OLV_OK;
+}
+
 }  // namespace olv
 
 using namespace olv;
@@ -296,37 +345,7 @@ int olv_graph_create(const uint32_t *rowptr, const uint32_t *col, const void *we
     int r = copy_in(g->rowptr, rowptr, ((size_t)V + 1) * 4, g->stream);
     if (r == OLV_OK) r = copy_in(g->col, col, E * 4, g->stream);
     if (r == OLV_OK && weight_type != OLV_W_NONE) r = copy_in(g->w, weights, E * 4, g->stream);
-    if (r == OLV_OK) {
-        // validate: rowptr monotone, rowptr[V] == E, col < V
-        std::vector<uint32_t> h(V + 1);
-        cudaError_t e = cudaMemcpyAsync(h.data(), g->rowptr.p, ((size_t)V + 1) * 4,
-                                        cudaMemcpyDeviceToHost, g->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-        if (e != cudaSuccess) r = cuda_fail(e, "rowptr check", __FILE__, __LINE__);
-        if (r == OLV_OK && (h[0] != 0 || h[V] != E)) {
-            set_error("olv_graph_create: rowptr[0]=%u rowptr[V]=%u, expected 0 and E=%llu",
-                      h[0], h[V], (unsigned long long)E);
-            r = OLV_ERR_ARG;
-        }
-        for (uint32_t v = 0; r == OLV_OK && v < V; v++)
-            if (h[v + 1] < h[v]) {
-                set_error("olv_graph_create: rowptr decreases at vertex %u", v);
-                r = OLV_ERR_ARG;
-            }
-    }
-    if (r == OLV_OK && E) {
-        std::vector<uint32_t> hc(E);
-        cudaError_t e = cudaMemcpyAsync(hc.data(), g->col.p, E * 4, cudaMemcpyDeviceToHost,
-                                        g->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
-        if (e != cudaSuccess) r = cuda_fail(e, "col check", __FILE__, __LINE__);
-        for (uint64_t i = 0; r == OLV_OK && i < E; i++)
-            if (hc[i] >= V) {
-                set_error("olv_graph_create: col[%llu]=%u out of range (V=%u)",
-                          (unsigned long long)i, hc[i], V);
-                r = OLV_ERR_ARG;
-            }
-    }
+    if (r == OLV_OK) r = check_csr(g);
     if (r == OLV_OK) r = finish_graph(g);
     if (r != OLV_OK) {
         olv_graph_destroy(g);

@@ -62,6 +62,7 @@
 #include "olive_b200/olv_advance.cuh"
 #include "olv_graphexec.cuh"
 #include "olv_internal.cuh"
+#include "olv_rowsolve.cuh"
 #include "olv_small.cuh"
 
 namespace olv {
@@ -1403,37 +1404,6 @@ static int sssp_relabel(olv_graph *g) {
     const uint32_t V = g->V;
     const uint64_t E = g->E;
     cudaStream_t s = g->stream;
-    std::vector<uint32_t> rp((size_t)V + 1), cp((size_t)V + 1);
-    OLV_CUDA(cudaMemcpyAsync(rp.data(), g->rowptr.p, ((size_t)V + 1) * 4, cudaMemcpyDeviceToHost, s));
-    OLV_CUDA(cudaMemcpyAsync(cp.data(), g->colptr.p, ((size_t)V + 1) * 4, cudaMemcpyDeviceToHost, s));
-    OLV_CUDA(cudaStreamSynchronize(s));
-    uint32_t maxd = 0;
-    for (uint32_t v = 0; v < V; v++) maxd = std::max(maxd, cp[v + 1] - cp[v]);
-    std::vector<uint64_t> start((size_t)maxd + 2, 0);
-    for (uint32_t v = 0; v < V; v++) start[maxd - (cp[v + 1] - cp[v]) + 1]++;
-    for (size_t d = 1; d < start.size(); d++) start[d] += start[d - 1];
-    std::vector<uint32_t> perm(V), newid(V), nrp((size_t)V + 1), ncp((size_t)V + 1);
-    for (uint32_t v = 0; v < V; v++) {
-        const uint32_t i = (uint32_t)start[maxd - (cp[v + 1] - cp[v])]++;
-        perm[i] = v;
-        newid[v] = i;
-    }
-    // in-degree > 0, and > 4, 8, 16, 32 (the pull's short-row bounds):
-    // prefixes of the new numbering
-    uint32_t vnz = 0, vlong[4] = {0, 0, 0, 0};
-    for (uint32_t v = 0; v < V; v++) {
-        const uint32_t din = cp[v + 1] - cp[v];
-        vnz += din != 0;
-        for (int k = 0; k < 4; k++) vlong[k] += din > (4u << k);
-    }
-    ws.sr_vnz = vnz;
-    for (int k = 0; k < 4; k++) ws.sr_vlong[k] = vlong[k];
-    nrp[0] = 0;
-    ncp[0] = 0;
-    for (uint32_t i = 0; i < V; i++) {
-        nrp[i + 1] = nrp[i] + (rp[perm[i] + 1] - rp[perm[i]]);
-        ncp[i + 1] = ncp[i] + (cp[perm[i] + 1] - cp[perm[i]]);
-    }
     OLV_TRY(ws.sr_perm.ensure((size_t)V * 4 + 16));
     OLV_TRY(ws.sr_newid.ensure((size_t)V * 4 + 16));
     OLV_TRY(ws.sr_rowptr.ensure(((size_t)V + 1) * 4 + 16));
@@ -1443,10 +1413,17 @@ static int sssp_relabel(olv_graph *g) {
     OLV_TRY(ws.sr_rowidx.ensure(E * 4 + 16));
     OLV_TRY(ws.sr_cw.ensure(E * 4 + 16));
     OLV_TRY(ws.sr_dist.ensure((size_t)V * 4 + 16));
-    OLV_CUDA(cudaMemcpyAsync(ws.sr_perm.p, perm.data(), (size_t)V * 4, cudaMemcpyHostToDevice, s));
-    OLV_CUDA(cudaMemcpyAsync(ws.sr_newid.p, newid.data(), (size_t)V * 4, cudaMemcpyHostToDevice, s));
-    OLV_CUDA(cudaMemcpyAsync(ws.sr_rowptr.p, nrp.data(), ((size_t)V + 1) * 4, cudaMemcpyHostToDevice, s));
-    OLV_CUDA(cudaMemcpyAsync(ws.sr_colptr.p, ncp.data(), ((size_t)V + 1) * 4, cudaMemcpyHostToDevice, s));
+    // by in-degree, highest first: in-degree > 0, and > 4, 8, 16, 32 (the pull's
+    // short-row bounds) are prefixes of the new numbering
+    OLV_TRY(sort_rows(g->colptr.as<uint32_t>(), V, s, ws.sr_perm.as<uint32_t>(),
+                      ws.sr_newid.as<uint32_t>(), ws.sr_colptr.as<uint32_t>()));
+    OLV_TRY(permuted_offsets(g->rowptr.as<uint32_t>(), ws.sr_perm.as<uint32_t>(), V, s,
+                             ws.sr_rowptr.as<uint32_t>()));
+    const uint32_t bounds[5] = {0, 4, 8, 16, 32};
+    uint32_t longer[5];
+    OLV_TRY(rows_longer(ws.sr_colptr.as<uint32_t>(), V, bounds, 5, s, longer));
+    ws.sr_vnz = longer[0];
+    std::copy(longer + 1, longer + 5, ws.sr_vlong);
     if (E) {
         k_sssp_relabel<<<g->num_sms * 16, kBlock, 0, s>>>(
             g->rowptr.as<uint32_t>(), g->col.as<uint32_t>(), g->w.as<uint32_t>(),
@@ -1458,7 +1435,6 @@ static int sssp_relabel(olv_graph *g) {
             ws.sr_rowidx.as<uint32_t>(), ws.sr_cw.as<uint32_t>());
         OLV_CUDA(cudaGetLastError());
     }
-    OLV_CUDA(cudaStreamSynchronize(s));   // the host vectors die here
     ws.sr_built = 1;
     return OLV_OK;
 }
