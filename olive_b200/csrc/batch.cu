@@ -2,8 +2,8 @@
 // run by ONE persistent kernel with a device-side work queue (no reference
 // counterpart; each instance's result equals its solo run, bit for bit).
 //
-// Work items are (instance, task) pairs handed out by an atomic counter,
-// largest instances first.  A CTA runs its item to completion:
+// Work items are (instance, task) pairs handed out by atomic counters,
+// largest instances first; the CTA or cluster that takes one runs it to completion:
 //   BFS from the instance's local vertex 0 (testBFS.cu semantics, levels
 //     relative to the instance, 0x7fffffff unreached).  The visited, current
 //     and next frontier bitmaps of the instance live in shared memory
@@ -11,14 +11,13 @@
 //     frontier with shared-memory atomicOr claims.
 //   PPR: K <= 32 personalised PageRank vectors with one-hot seeds (the
 //     oracle's orc_ppr definition: dangling mass returns to the seed), pulled
-//     over the in-edges with one warp per vertex and lane k = vector k, so
-//     each in-edge reads one 128-byte row, scaled by the source's inverse
-//     out-degree (computed once per item).  A warp keeps eight rows in
-//     flight; sums still run in CSC order per lane, the dangling mass is
-//     summed while the new vectors are written, and cross-warp reductions
-//     run in a fixed order, so results do not depend on which CTA runs the
-//     item or when.  Stops after max_it iterations or when every vector's L1
-//     change (FP64) is below tol.
+//     over the in-edges, summed in CSC order per vertex and vector.  K = 4, 8,
+//     16 or 32: a lane owns four vectors, so one warp gathers for 32 / (K / 4)
+//     vertices at a time; any other K: one warp per vertex, lane k = vector k.
+//     The dangling mass is summed while the new vectors are written, in an
+//     order-free or a fixed way, so results do not depend on which CTA runs
+//     the item or when.  Stops after max_it iterations or when every vector's
+//     L1 change (FP64) is below tol.
 #include <algorithm>
 #include <numeric>
 #include <vector>
@@ -35,6 +34,13 @@ namespace olv {
 constexpr int kBatchThreads = 512;
 constexpr uint32_t kBatchMaxV = 65536;
 constexpr int kBatchWarps = kBatchThreads / 32;
+constexpr int kBatchMaxWarps = 32;
+// PPR items of at most this many vertices take one CTA, larger ones a cluster: a
+// sweep of a small instance on 16 CTAs is mostly its barrier, while a larger one on a
+// CTA is left running alone at the end.  The line at 512 / 1024 / 2048 / 4096, K = 32,
+// 20 sweeps: 512 instances of 50..2000 vertices 5.5 / 4.1 / 2.0 / - ms, 64 of 300..9001
+// 1.88 / 1.94 / 2.31 / 2.65, 96 of 1024..65536 11.6 / 11.6 / 11.6 / 12.5.
+constexpr uint32_t kCtaItem = 2048;
 
 struct BatchArgs {
     const uint32_t *rowptr, *col, *colptr, *rowidx;
@@ -48,6 +54,8 @@ struct BatchArgs {
     int32_t *levels;             // [V]
     float *ppr, *ppr_tmp;        // [V][K]
     float *inv_deg;              // [V] 1 / out-degree (0: dangling), written per PPR item
+    uint2 *ew;                   // [E] in-edges as (local source, its inverse degree), K % 4 == 0
+    uint32_t n_large;            // items order[0 .. n_large) are a cluster's, the rest a CTA's
     uint32_t *counter;           // work queue head
     uint32_t *ppr_iters;         // [count]
     unsigned long long *stats;   // [0] BFS edges traversed, [1] PPR edge visits, [2] error bits
@@ -208,138 +216,238 @@ __device__ __forceinline__ void ppr_sweep_warp(const BatchArgs &a, const PprView
     }
 }
 
-#ifndef OLV_QROUND
-#define OLV_QROUND 4
-#endif
-constexpr int kQRound = OLV_QROUND;   // in-edges per vertex gathered per round
+// ---- rows of four vectors per lane (K = 4, 8, 16 or 32) --------------------
+// L = K / 4 lanes per vertex, a float4 of vectors per lane, so a warp sweeps
+// 32 / L vertices at once.  In-edges are read as (source, inverse degree) pairs
+// laid out once per item: every lane of a vertex loads the pair itself (one
+// broadcast load, no index arithmetic or shuffles), four pairs ahead of the four
+// rows being gathered.  A place past a vertex's in-edges
+// weighs zero.  Every vertex's in-edges are folded in CSC order.  The dangling
+// mass is summed in 64-bit fixed point (units of 2^-62; the masses of a vector
+// sum to at most one), so it does not depend on which warp adds what when; the
+// L1 change (FP64, only with a tolerance to compare it with) is combined in a
+// fixed order.
+// The sweep this replaces (one chunk of indices per vertex, sources and weights
+// by shuffles, K = 32 only) took 690 warp instructions per four vertices of eight
+// in-edges and was bound by them: 96 uniform digraphs of 1024..65536 vertices,
+// K = 32, 20 sweeps 18.0 -> 11.6 ms; K = 8 (a lane per vector before) 30.4 -> 5.8 ms.
+constexpr double kDangOne = 4611686018427387904.0;   // 2^62
 
-// K = 32 sweep with four vertices per warp: slot s = lane >> 3 (8 lanes)
-// takes vertex 4g + s of vertex group g (g = w0, w0 + nw, ...), lane quad q =
-// lane & 7 holds vectors 4q .. 4q+3 of it as one float4.  A round gathers
-// two in-edges of each of the four vertices (one 16-byte load per lane per
-// in-edge), so the per-vertex work -- offsets, sources, update, residual --
-// is shared by four vertices per instruction.  Each vertex's in-edges are
-// folded in CSC order; the warp's dangling mass and L1 change are combined
-// over the slots by a fixed shuffle tree and returned in the lane-per-vector
-// layout, like ppr_sweep_warp.  `visits` gets the warp's in-edge visits.
-// Needs 16-byte aligned vectors.  Used by the cluster kernel, whose rows come
-// from L2 (the one-CTA-per-item kernel is bound by DRAM traffic and keeps the
-// 4-byte path).
-__device__ __forceinline__ void ppr_sweep_warp_q(const BatchArgs &a, const PprView &p,
-                                                 uint32_t lane, uint32_t w0, uint32_t nw,
-                                                 const float *src, float *dst, float dk,
-                                                 float &dpart, double &res,
-                                                 unsigned long long &visits) {
-    constexpr unsigned kFull = 0xffffffffu;
-    const uint32_t base = p.base, n = p.n;
-    const uint32_t slot = lane >> 3, quad = lane & 7;
-    const float4 *src4 = reinterpret_cast<const float4 *>(src);
-    float4 *dst4 = reinterpret_cast<float4 *>(dst);
-    uint32_t seed4[4];
-    float dk4[4];
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-        seed4[c] = __shfl_sync(kFull, p.seed, 4 * quad + c);
-        dk4[c] = __shfl_sync(kFull, dk, 4 * quad + c);
-    }
-    float dp4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    double rs4[4] = {0.0, 0.0, 0.0, 0.0};
-    unsigned long long vq = 0;
-    for (uint32_t g = w0; 4 * g < n; g += nw) {
-        const uint32_t v = 4 * g + slot;
+struct alignas(16) RowsShared {
+    unsigned long long dang[3][32];       // this CTA's dangling mass, by sweep modulo 3
+    double warp_res[kBatchMaxWarps][32];  // per warp and vector
+    double res[2][32];                    // this CTA's L1 change, by sweep parity
+    alignas(16) uint32_t seed[32];
+    alignas(16) float tele[32];           // what a seed gets in this sweep
+    int stop;
+};
+
+// One sweep of one warp over the vertex groups g = w0, w0 + nw, ...; adds the new
+// dangling mass to dang (shared) and, kRes, the L1 change to res.
+template <int L, bool kRes>
+__device__ __forceinline__ void ppr_sweep_rows(const BatchArgs &a, const PprView &p,
+                                               const RowsShared &sh, uint32_t lane, uint32_t w0,
+                                               uint32_t nw, const float *src, float *dst,
+                                               unsigned long long *dang, double (&res)[4]) {
+    constexpr uint32_t kVerts = 32 / L;
+    const uint32_t slot = lane / L, q = lane % L, n = p.n;
+    const float4 *src4 = reinterpret_cast<const float4 *>(src) + q;
+    float4 *dst4 = reinterpret_cast<float4 *>(dst) + q;
+    for (uint32_t g = w0; g * kVerts < n; g += nw) {
+        const uint32_t v = g * kVerts + slot;
         const bool valid = v < n;
         uint32_t b = 0, deg = 0;
+        float inv = 1.0f;
+        float4 old;
         if (valid) {
-            b = a.colptr[base + v];
-            deg = a.colptr[base + v + 1] - b;
+            b = a.colptr[p.base + v];
+            deg = a.colptr[p.base + v + 1] - b;
+            inv = p.inv[v];
+            if (kRes) old = src4[(size_t)v * L];
         }
-        uint32_t maxdeg = deg;
-        maxdeg = max(maxdeg, __shfl_xor_sync(kFull, maxdeg, 8));
-        maxdeg = max(maxdeg, __shfl_xor_sync(kFull, maxdeg, 16));
+        const uint32_t longest = __reduce_max_sync(0xffffffffu, deg);
+        const uint2 *ew = a.ew + b;
+        uint2 e[4];
+#pragma unroll
+        for (uint32_t r = 0; r < 4; r++) e[r] = r < deg ? ew[r] : make_uint2(0u, 0u);
         float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        for (uint32_t c0 = 0; c0 < maxdeg; c0 += 8) {
-            // lane quad q of a slot holds in-edge c0 + q of the slot's vertex
-            uint32_t u = 0;
-            float w = 0.0f;
-            if (c0 + quad < deg) {
-                u = a.rowidx[b + c0 + quad] - base;
-                if (u >= n) {   // edge enters from outside the instance
-                    atomicOr((unsigned int *)&a.stats[2], 2u);
-                    u = 0;
-                } else {
-                    w = p.inv[u];
-                }
+        for (uint32_t c = 0; c < longest; c += 4) {
+            float4 x[4];
+            float w[4];
+#pragma unroll
+            for (uint32_t r = 0; r < 4; r++) {
+                x[r] = src4[(size_t)e[r].x * L];
+                w[r] = __uint_as_float(e[r].y);
             }
-            const uint32_t cend = min(8u, maxdeg - c0);
-            for (uint32_t t = 0; t < cend; t += kQRound) {
-                float4 x[kQRound];
-                float wj[kQRound];
 #pragma unroll
-                for (int r = 0; r < kQRound; r++) {
-                    const uint32_t i = t + r;
-                    const uint32_t uj = __shfl_sync(kFull, u, slot * 8 + (i & 7));
-                    wj[r] = __shfl_sync(kFull, w, slot * 8 + (i & 7));
-                    x[r] = c0 + i < deg ? src4[(size_t)uj * 8 + quad]
-                                        : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                }
+            for (uint32_t r = 0; r < 4; r++)
+                e[r] = c + 4 + r < deg ? ew[c + 4 + r] : make_uint2(0u, 0u);
 #pragma unroll
-                for (int r = 0; r < kQRound; r++) {
-                    if (c0 + t + r < deg) {
-                        acc.x = fmaf(x[r].x, wj[r], acc.x);
-                        acc.y = fmaf(x[r].y, wj[r], acc.y);
-                        acc.z = fmaf(x[r].z, wj[r], acc.z);
-                        acc.w = fmaf(x[r].w, wj[r], acc.w);
-                    }
-                }
+            for (uint32_t r = 0; r < 4; r++) {
+                acc.x = fmaf(x[r].x, w[r], acc.x);
+                acc.y = fmaf(x[r].y, w[r], acc.y);
+                acc.z = fmaf(x[r].z, w[r], acc.z);
+                acc.w = fmaf(x[r].w, w[r], acc.w);
             }
         }
-        if (quad == 0) vq += deg;
         if (valid) {
-            const float4 old = src4[(size_t)v * 8 + quad];
-            const float a4[4] = {acc.x, acc.y, acc.z, acc.w};
-            const float o4[4] = {old.x, old.y, old.z, old.w};
-            float nv[4];
-            const bool dang = p.inv[v] == 0.0f;
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                const float tele = (v == seed4[c]) ? fmaf(p.alpha, dk4[c], 1.0f - p.alpha) : 0.0f;
-                nv[c] = fmaf(p.alpha, a4[c], tele);
-                rs4[c] += fabs((double)nv[c] - (double)o4[c]);
-                if (dang) dp4[c] += nv[c];
+            const uint4 sd = reinterpret_cast<const uint4 *>(sh.seed)[q];
+            float4 t = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (sd.x == v || sd.y == v || sd.z == v || sd.w == v) {
+                const float4 s = reinterpret_cast<const float4 *>(sh.tele)[q];
+                t = make_float4(sd.x == v ? s.x : 0.0f, sd.y == v ? s.y : 0.0f,
+                                sd.z == v ? s.z : 0.0f, sd.w == v ? s.w : 0.0f);
             }
-            dst4[(size_t)v * 8 + quad] = make_float4(nv[0], nv[1], nv[2], nv[3]);
+            const float4 nv = make_float4(fmaf(p.alpha, acc.x, t.x), fmaf(p.alpha, acc.y, t.y),
+                                          fmaf(p.alpha, acc.z, t.z), fmaf(p.alpha, acc.w, t.w));
+            if (kRes) {
+                res[0] += fabs((double)nv.x - (double)old.x);
+                res[1] += fabs((double)nv.y - (double)old.y);
+                res[2] += fabs((double)nv.z - (double)old.z);
+                res[3] += fabs((double)nv.w - (double)old.w);
+            }
+            dst4[(size_t)v * L] = nv;
+            if (inv == 0.0f) {   // a dangling vertex: rare enough for shared atomics
+                atomicAdd(&dang[4 * q], __double2ull_rn((double)nv.x * kDangOne));
+                atomicAdd(&dang[4 * q + 1], __double2ull_rn((double)nv.y * kDangOne));
+                atomicAdd(&dang[4 * q + 2], __double2ull_rn((double)nv.z * kDangOne));
+                atomicAdd(&dang[4 * q + 3], __double2ull_rn((double)nv.w * kDangOne));
+            }
         }
     }
-    // slots 0+1 and 2+3, then the pairs; back to lane k = vector k
-#pragma unroll
-    for (int o = 8; o <= 16; o <<= 1) {
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            dp4[c] += __shfl_xor_sync(kFull, dp4[c], o);
-            rs4[c] += __shfl_xor_sync(kFull, rs4[c], o);
-        }
-        vq += __shfl_xor_sync(kFull, vq, o);
-    }
-    const uint32_t from = lane >> 2, comp = lane & 3;
-    float dsel = 0.0f;
-    double rsel = 0.0;
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-        const float dc = __shfl_sync(kFull, dp4[c], from);
-        const double rc = __shfl_sync(kFull, rs4[c], from);
-        if (comp == (uint32_t)c) {
-            dsel = dc;
-            rsel = rc;
-        }
-    }
-    dpart += dsel;
-    res += rsel;
-    visits += vq;
 }
 
-// Whether an item's sweeps can use the 16-byte row path.
-__device__ __forceinline__ bool ppr_v4(const BatchArgs &a) {
-    return a.K == 32 && ((reinterpret_cast<uintptr_t>(a.ppr) | reinterpret_cast<uintptr_t>(a.ppr_tmp)) & 15) == 0;
+// A PPR item by a team of C CTAs (this is CTA `rank`); sync(): the team's barrier,
+// at(p, r): CTA r's copy of a shared variable.
+template <int L, class Sync, class At>
+__device__ void team_ppr(const BatchArgs &a, uint32_t inst, uint32_t C, uint32_t rank, Sync sync,
+                         At at, RowsShared &sh) {
+    constexpr unsigned kFull = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const uint32_t gw = rank * warps + wid, nw = C * warps, q = lane % L;
+    const PprView p = ppr_view(a, inst, lane);
+    const bool with_res = a.tol > 0.0;   // nothing is below a tolerance of zero
+    // start vectors and inverse degrees, then the in-edges as pairs
+    const uint32_t tid = rank * blockDim.x + threadIdx.x, nt = C * blockDim.x;
+    for (uint32_t v = tid; v < p.n; v += nt) {
+        const uint32_t deg = a.rowptr[p.base + v + 1] - a.rowptr[p.base + v];
+        p.inv[v] = deg ? __fdiv_rn(1.0f, (float)deg) : 0.0f;
+    }
+    for (uint32_t i = tid; i < p.n * L; i += nt) {
+        const uint32_t v = i / L, k = 4 * (i % L);
+        const uint32_t *sd = a.seeds + (size_t)inst * p.K + k;
+        reinterpret_cast<float4 *>(p.r0)[i] =
+            make_float4(v == sd[0] ? 1.0f : 0.0f, v == sd[1] ? 1.0f : 0.0f,
+                        v == sd[2] ? 1.0f : 0.0f, v == sd[3] ? 1.0f : 0.0f);
+    }
+    // dangling mass of the start: the seeds without out-edges (counted by CTA 0)
+    if (threadIdx.x < 32) {
+        unsigned long long d = 0;
+        if (rank == 0 && (int)lane < p.K) {
+            const uint32_t s = p.base + p.seed;
+            if (a.rowptr[s + 1] == a.rowptr[s]) d = (unsigned long long)kDangOne;
+        }
+        sh.dang[0][lane] = d;
+        sh.dang[1][lane] = 0;
+        sh.seed[lane] = p.seed;   // ~0 past the K vectors
+    }
+    sync();
+    const uint64_t e0 = a.colptr[p.base], e1 = a.colptr[p.base + p.n];
+    for (uint64_t e = e0 + tid; e < e1; e += nt) {
+        uint32_t u = a.rowidx[e] - p.base;
+        float w = 0.0f;
+        if (u >= p.n) {   // edge enters from outside the instance
+            atomicOr((unsigned int *)&a.stats[2], 2u);
+            u = 0;
+        } else {
+            w = p.inv[u];
+        }
+        a.ew[e] = make_uint2(u, __float_as_uint(w));
+    }
+    sync();
+    int it = 0;
+    while (it < a.max_it) {
+        const int pb = it & 1;
+        if (threadIdx.x < 32) {   // every CTA adds the team's masses (integers: in any order)
+            unsigned long long t = 0;
+            for (uint32_t r = 0; r < C; r++) t += at(&sh.dang[it % 3][0], r)[lane];
+            sh.tele[lane] = fmaf(p.alpha, (float)((double)t / kDangOne), 1.0f - p.alpha);
+            sh.dang[(it + 2) % 3][lane] = 0;   // read in the last sweep, added to in the next
+        }
+        __syncthreads();
+        const float *src = pb ? p.r1 : p.r0;
+        float *dst = pb ? p.r0 : p.r1;
+        unsigned long long *dang = sh.dang[(it + 1) % 3];
+        double res[4] = {0.0, 0.0, 0.0, 0.0};
+        if (with_res)
+            ppr_sweep_rows<L, true>(a, p, sh, lane, gw, nw, src, dst, dang, res);
+        else
+            ppr_sweep_rows<L, false>(a, p, sh, lane, gw, nw, src, dst, dang, res);
+        if (with_res) {
+            // the warp's slots by a fixed tree, then the CTA's warps in order
+#pragma unroll
+            for (int o = L; o < 32; o <<= 1)
+#pragma unroll
+                for (int c = 0; c < 4; c++) res[c] += __shfl_xor_sync(kFull, res[c], o);
+            if (lane < L)
+#pragma unroll
+                for (int c = 0; c < 4; c++) sh.warp_res[wid][4 * q + c] = res[c];
+            __syncthreads();
+            if (wid == 0) {
+                double t = 0.0;
+                if ((int)lane < p.K)
+                    for (uint32_t w = 0; w < warps; w++) t += sh.warp_res[w][lane];
+                sh.res[pb][lane] = t;
+            }
+        }
+        // orders this sweep's writes (vectors and sums) before the next sweep's reads
+        sync();
+        it++;
+        if (with_res) {   // stop test: the same on every CTA
+            if (wid == 0) {
+                double t = 0.0;
+                for (uint32_t r = 0; r < C; r++) t += at(&sh.res[pb][0], r)[lane];
+                double mx = (int)lane < p.K ? t : 0.0;
+#pragma unroll
+                for (int o = 16; o; o >>= 1) mx = fmax(mx, __shfl_xor_sync(kFull, mx, o));
+                if (lane == 0) sh.stop = mx < a.tol;
+            }
+            __syncthreads();
+            if (sh.stop) break;
+        }
+    }
+    if (it & 1) {   // result is in the scratch copy
+        for (uint32_t i = tid; i < p.n * L; i += nt)
+            reinterpret_cast<float4 *>(p.r0)[i] = reinterpret_cast<const float4 *>(p.r1)[i];
+    }
+    if (tid == 0) {
+        a.ppr_iters[inst] = it;
+        atomicAdd(&a.stats[1], (unsigned long long)(e1 - e0) * (unsigned long long)it *
+                                   (unsigned long long)p.K);
+    }
+    sync();   // shared state and vectors are the next item's
+}
+
+// Whether an item's sweeps can use rows of four vectors per lane.
+__device__ __forceinline__ bool ppr_rows(const BatchArgs &a) {
+    return a.ew != nullptr;
+}
+
+template <class Sync, class At>
+__device__ __forceinline__ void team_ppr_k(const BatchArgs &a, uint32_t inst, uint32_t C,
+                                           uint32_t rank, Sync sync, At at, RowsShared &sh) {
+    switch (a.K) {
+        case 32: team_ppr<8>(a, inst, C, rank, sync, at, sh); break;
+        case 16: team_ppr<4>(a, inst, C, rank, sync, at, sh); break;
+        case 8: team_ppr<2>(a, inst, C, rank, sync, at, sh); break;
+        default: team_ppr<1>(a, inst, C, rank, sync, at, sh); break;
+    }
+}
+
+// The same by this CTA alone.
+__device__ __forceinline__ void cta_rows_ppr(const BatchArgs &a, uint32_t inst, RowsShared &sh) {
+    team_ppr_k(
+        a, inst, 1, 0, [] { __syncthreads(); }, [](auto *p, uint32_t) { return p; }, sh);
 }
 
 __device__ void cta_ppr(const BatchArgs &a, uint32_t inst) {
@@ -397,6 +505,7 @@ __device__ void cta_ppr(const BatchArgs &a, uint32_t inst) {
 
 __global__ void __launch_bounds__(kBatchThreads) k_batch(BatchArgs a) {
     __shared__ uint32_t bm[3 * (kBatchMaxV / 32)];
+    __shared__ RowsShared rows;
     __shared__ uint32_t s_item;
     const uint32_t n_items = (uint32_t)a.count * a.tasks;
     for (;;) {
@@ -409,22 +518,22 @@ __global__ void __launch_bounds__(kBatchThreads) k_batch(BatchArgs a) {
         const bool bfs = a.tasks == 2 ? (item % 2 == 0) : (a.do_bfs != 0);
         if (bfs)
             cta_bfs(a, inst, bm);
+        else if (ppr_rows(a))
+            cta_rows_ppr(a, inst, rows);
         else
             cta_ppr(a, inst);
     }
 }
 
 // ---- cluster version ------------------------------------------------------
-// The same items, with every PPR item run by a whole thread-block cluster
+// The same items, with the larger PPR items run by a whole thread-block cluster
 // (16 CTAs of 1024 threads where the GPU allows it, else 8): the cluster's
 // 512 (256) warps split the instance's vertices, and the per-iteration
 // reductions go through distributed shared memory with one cluster barrier
 // per iteration.  Only a handful of instances are in flight at a time, so
-// their PPR vectors (2 x V_i x 128 B each) stay in L2 and the 128-byte row
-// gathers, eight per vertex per iteration, hit L2 instead of DRAM.  BFS items
-// still take one CTA each, before the PPR items.  Results depend on the
-// cluster size (it fixes the order of the dangling-mass sums), never on
-// scheduling: a solo run with the same cluster size is bitwise equal.
+// their PPR vectors (2 x V_i x 128 B each) stay in L2 and the row gathers
+// hit L2 instead of DRAM.  A solo run with the same cluster size is bitwise
+// equal: nothing depends on scheduling.
 constexpr int kClusterThreads = 1024;
 constexpr int kClusterWarps = kClusterThreads / 32;
 
@@ -463,10 +572,7 @@ __device__ void cluster_ppr(const BatchArgs &a, uint32_t inst, cg::cluster_group
         float *dst = pb ? p.r0 : p.r1;
         double res = 0.0;
         float dpart = 0.0f;
-        if (ppr_v4(a))
-            ppr_sweep_warp_q(a, p, lane, gw, nw, src, dst, dk, dpart, res, visits);
-        else
-            ppr_sweep_warp(a, p, lane, gw, nw, src, dst, dk, dpart, res, visits);
+        ppr_sweep_warp(a, p, lane, gw, nw, src, dst, dk, dpart, res, visits);
         sh.d[wid][lane] = dpart;
         sh.res[wid][lane] = res;
         __syncthreads();
@@ -505,9 +611,38 @@ __device__ void cluster_ppr(const BatchArgs &a, uint32_t inst, cg::cluster_group
 
 __global__ void __launch_bounds__(kClusterThreads, 1) k_batch_cluster(BatchArgs a) {
     __shared__ uint32_t bm[3 * (kBatchMaxV / 32)];
-    __shared__ ClusterShared sh;
+    __shared__ union {
+        ClusterShared one;   // a lane per vector
+        RowsShared rows;     // four vectors per lane
+    } sh;
     __shared__ uint32_t s_item;
     cg::cluster_group cl = cg::this_cluster();
+    // the cluster's items first, largest first (counter[1], taken by CTA 0), then
+    // the CTA's, then BFS: the smaller ones level the CTAs' ends
+    if (a.do_ppr) {
+        for (;;) {
+            if (cl.block_rank() == 0 && threadIdx.x == 0) s_item = atomicAdd(&a.counter[1], 1u);
+            cl.sync();
+            const uint32_t item = *cl.map_shared_rank(&s_item, 0);
+            if (item >= a.n_large) break;
+            if (ppr_rows(a))
+                team_ppr_k(
+                    a, a.order[item], cl.num_blocks(), cl.block_rank(), [&] { cl.sync(); },
+                    [&](auto *p, uint32_t r) { return cl.map_shared_rank(p, r); }, sh.rows);
+            else
+                cluster_ppr(a, a.order[item], cl, sh.one);
+        }
+        cl.sync();   // the last item's number has been read by every CTA
+        for (;;) {
+            __syncthreads();
+            if (threadIdx.x == 0) s_item = a.n_large + atomicAdd(&a.counter[2], 1u);
+            __syncthreads();
+            const uint32_t item = s_item;
+            if (item >= (uint32_t)a.count) break;
+            cta_rows_ppr(a, a.order[item], sh.rows);
+        }
+        __syncthreads();
+    }
     if (a.do_bfs) {   // BFS items: one CTA each (counter[0])
         for (;;) {
             if (threadIdx.x == 0) s_item = atomicAdd(&a.counter[0], 1u);
@@ -516,15 +651,6 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_batch_cluster(BatchArgs 
             __syncthreads();
             if (item >= (uint32_t)a.count) break;
             cta_bfs(a, a.order[item], bm);
-        }
-    }
-    if (a.do_ppr) {   // PPR items: one cluster each (counter[1], taken by CTA 0)
-        for (;;) {
-            if (cl.block_rank() == 0 && threadIdx.x == 0) s_item = atomicAdd(&a.counter[1], 1u);
-            cl.sync();
-            const uint32_t item = *cl.map_shared_rank(&s_item, 0);
-            if (item >= (uint32_t)a.count) break;
-            cluster_ppr(a, a.order[item], cl, sh);
         }
     }
     cl.sync();   // no CTA leaves while another may still read its shared memory
@@ -570,9 +696,10 @@ static int launch_batch_cluster(const BatchArgs &a, int num_sms, cudaStream_t s,
 // Device buffers of olv_batch_run, kept with the graph between calls (they
 // only grow), so a call allocates nothing once the sizes have been seen.
 struct BatchState {
-    DevBuf off, order, seeds, tmp, inv, counter, iters, stats, levels, ppr;
+    DevBuf off, order, seeds, tmp, inv, ew, counter, iters, stats, levels, ppr;
     ~BatchState() {
-        off.release(); order.release(); seeds.release(); tmp.release(); inv.release(); counter.release();
+        off.release(); order.release(); seeds.release(); tmp.release(); inv.release(); ew.release();
+        counter.release();
         iters.release(); stats.release(); levels.release(); ppr.release();
     }
 };
@@ -671,6 +798,21 @@ extern "C" int olv_batch_run(olv_graph *g, const uint32_t *inst_offsets, int cou
     a.ppr = ppr_out ? (dev_pr ? ppr_out : bs.ppr.as<float>()) : nullptr;
     a.ppr_tmp = bs.tmp.as<float>();
     a.inv_deg = bs.inv.as<float>();
+    // rows of four vectors per lane need whole 16-byte rows
+    bool rows = ppr_out && (K == 4 || K == 8 || K == 16 || K == 32) &&
+                (((uintptr_t)a.ppr | (uintptr_t)a.ppr_tmp) & 15) == 0;
+    if (rows && bs.ew.ensure(g->E * 8 + 16) != OLV_OK) {   // no room for the pairs
+        cudaGetLastError();
+        rows = false;
+    }
+    a.ew = rows ? bs.ew.as<uint2>() : nullptr;
+    a.n_large = (uint32_t)count;
+    if (rows) {
+        a.n_large = 0;
+        while (a.n_large < (uint32_t)count &&
+               off[order[a.n_large] + 1] - off[order[a.n_large]] > kCtaItem)
+            a.n_large++;
+    }
     a.counter = bs.counter.as<uint32_t>();
     a.ppr_iters = bs.iters.as<uint32_t>();
     a.stats = bs.stats.as<unsigned long long>();
