@@ -507,7 +507,12 @@ k_bfs_pull(const uint32_t *__restrict__ colptr, const uint32_t *__restrict__ row
 
 // Pull, pass 2: eight lanes per candidate probe in-edges 1..8 at once (one
 // 32-byte sector of the in-edge list).  A candidate with in-edges left after
-// that goes to the overflow list.
+// that goes to the overflow list.  The pass is a chain of dependent loads
+// (candidate, its range, its in-edges, the bitmap), so a warp takes 32
+// candidates, a lane each for all but the probes, and issues the eight rounds
+// of in-edge loads, then the eight of bitmap probes, together: 77 -> 27 us on the
+// widest pull level of a uniform digraph (1 M vertices, 8 M edges), where a warp
+// took four before.
 __global__ void __launch_bounds__(kBlock)
 k_bfs_pull_cand(const uint32_t *__restrict__ colptr, const uint32_t *__restrict__ rowptr,
                 TravCtl *c, PullLists p) {
@@ -518,37 +523,52 @@ k_bfs_pull_cand(const uint32_t *__restrict__ colptr, const uint32_t *__restrict_
     const int L = (int)c->level;
     const uint32_t *__restrict__ fin = c->fb_cur ? p.fb1 : p.fb0;
     uint32_t *fout = c->fb_cur ? p.fb0 : p.fb1;
-    const uint32_t lane = lane_id(), sub = lane & 7, grp = lane & 24;
+    const uint32_t lane = lane_id(), sub = lane & 7, grp = lane >> 3;
     const uint32_t gwarp = (blockIdx.x * kBlock + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * kBlock) >> 5;
+    constexpr int kRounds = 8;   // of four candidates
     unsigned long long acc = 0, nfound = 0;
-    for (uint64_t base = (uint64_t)gwarp * 4; base < n; base += (uint64_t)nwarps * 4) {
-        const uint64_t i = base + (lane >> 3);
-        const bool valid = i < n;
+    for (uint64_t base = (uint64_t)gwarp * 32; base < n; base += (uint64_t)nwarps * 32) {
+        const bool valid = base + lane < n;
         uint32_t v = 0, b = 0, e = 0;
         if (valid) {
-            v = p.cand[i];
+            v = p.cand[base + lane];
             b = __ldg(&colptr[v]) + 1;
             e = __ldg(&colptr[v + 1]);
         }
-        const uint32_t j = b + sub;
-        const bool hit = valid && j < e && in_bitmap(fin, __ldg(&p.pidx[j]));
-        const uint32_t gm = (__ballot_sync(0xffffffffu, hit) >> grp) & 0xffu;
-        const bool more = valid && !gm && e > b + kGroupProbe;
-        if (valid && gm && sub == 0) {
+        uint32_t u[kRounds];
+        bool on[kRounds];
+#pragma unroll
+        for (int r = 0; r < kRounds; r++) {
+            const uint32_t j = __shfl_sync(0xffffffffu, b, 4 * r + grp) + sub;
+            on[r] = j < __shfl_sync(0xffffffffu, e, 4 * r + grp);
+            u[r] = on[r] ? __ldg(&p.pidx[j]) : 0u;
+        }
+        uint32_t w[kRounds];
+#pragma unroll
+        for (int r = 0; r < kRounds; r++) w[r] = on[r] ? __ldg(&fin[u[r] >> 5]) : 0u;
+        bool hit = false;
+#pragma unroll
+        for (int r = 0; r < kRounds; r++) {
+            const uint32_t m = __ballot_sync(0xffffffffu, (w[r] >> (u[r] & 31)) & 1u);
+            if ((lane >> 2) == (uint32_t)r) hit = (m >> (8 * (lane & 3))) & 0xffu;
+        }
+        if (hit) {
             level[v] = L + 1;
             atomicOr(&fout[v >> 5], 1u << (v & 31));
             acc += __ldg(&rowptr[v + 1]) - __ldg(&rowptr[v]);
             nfound++;
         }
-        warp_push(more && sub == 0, v, p.ovf, &c->ncand[1]);
+        warp_push(valid && !hit && e > b + kGroupProbe, v, p.ovf, &c->ncand[1]);
     }
     warp_add64(acc, &c->m_next);
     warp_add64(nfound, &c->reached_pull);
 }
 
-// Pull, pass 3: one warp per overflow vertex scans the rest of its in-edges,
-// 32 per probe, and stops at the first parent.
+// Pull, pass 3: the rest of the overflow vertices' in-edges, up to the first
+// parent.  A warp takes four vertices: the first 32 in-edges of each are probed
+// together (the same chain of loads), then those of a vertex without a parent
+// yet 32 at a time.
 __global__ void __launch_bounds__(kBlock)
 k_bfs_pull_overflow(const uint32_t *__restrict__ colptr, const uint32_t *__restrict__ rowptr,
                     TravCtl *c, PullLists p) {
@@ -562,20 +582,35 @@ k_bfs_pull_overflow(const uint32_t *__restrict__ colptr, const uint32_t *__restr
     const uint32_t lane = lane_id();
     const uint32_t gwarp = (blockIdx.x * kBlock + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * kBlock) >> 5;
+    constexpr int kTake = 4;
     unsigned long long acc = 0, nfound = 0;
-    for (uint32_t i = gwarp; i < n; i += nwarps) {
-        const uint32_t v = p.ovf[i];
-        const uint32_t b = __ldg(&colptr[v]) + 1 + kGroupProbe, e = __ldg(&colptr[v + 1]);
-        bool found = false;
-        for (uint32_t base = b; base < e; base += 32) {
-            const uint32_t j = base + lane;
-            const bool hit = j < e && in_bitmap(fin, __ldg(&p.pidx[j]));
-            if (__any_sync(0xffffffffu, hit)) {
-                found = true;
-                break;
-            }
+    for (uint64_t first = gwarp; first < n; first += (uint64_t)nwarps * kTake) {
+        // lane t < kTake: vertex first + t * nwarps
+        const uint64_t i = first + (uint64_t)lane * nwarps;
+        uint32_t v = 0, b = 0, e = 0;
+        if (lane < kTake && i < n) {
+            v = p.ovf[i];
+            b = __ldg(&colptr[v]) + 1 + kGroupProbe;
+            e = __ldg(&colptr[v + 1]);
         }
-        if (lane == 0 && found) {
+        uint32_t u[kTake], bt[kTake], et[kTake], w[kTake];
+#pragma unroll
+        for (int t = 0; t < kTake; t++) {
+            bt[t] = __shfl_sync(0xffffffffu, b, t) + lane;
+            et[t] = __shfl_sync(0xffffffffu, e, t);
+            u[t] = bt[t] < et[t] ? __ldg(&p.pidx[bt[t]]) : 0u;
+        }
+#pragma unroll
+        for (int t = 0; t < kTake; t++) w[t] = bt[t] < et[t] ? __ldg(&fin[u[t] >> 5]) : 0u;
+        uint32_t found = 0;
+#pragma unroll
+        for (int t = 0; t < kTake; t++) {
+            bool hit = __any_sync(0xffffffffu, (w[t] >> (u[t] & 31)) & 1u);
+            for (uint32_t j = bt[t] + 32; !hit && j - lane < et[t]; j += 32)
+                hit = __any_sync(0xffffffffu, j < et[t] && in_bitmap(fin, __ldg(&p.pidx[j])));
+            found |= (uint32_t)hit << t;
+        }
+        if ((found >> lane) & 1u) {
             level[v] = L + 1;
             atomicOr(&fout[v >> 5], 1u << (v & 31));
             acc += __ldg(&rowptr[v + 1]) - __ldg(&rowptr[v]);
