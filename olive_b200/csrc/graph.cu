@@ -29,26 +29,6 @@ int cuda_fail(cudaError_t e, const char *what, const char *file, int line) {
     return e == cudaErrorMemoryAllocation ? OLV_ERR_NOMEM : OLV_ERR_CUDA;
 }
 
-int DevBuf::ensure(size_t n) {
-    if (n <= bytes && p) return OLV_OK;
-    release();
-    if (n == 0) n = 16;
-    cudaError_t e = cudaMalloc(&p, n);
-    if (e != cudaSuccess) {
-        p = nullptr;
-        bytes = 0;
-        return cuda_fail(e, "cudaMalloc", __FILE__, __LINE__);
-    }
-    bytes = n;
-    return OLV_OK;
-}
-
-void DevBuf::release() {
-    if (p) cudaFree(p);
-    p = nullptr;
-    bytes = 0;
-}
-
 int resident_blocks(const olv_graph *g, const void *kernel, int *blocks) {
     int per_sm = 0;
     OLV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBlock, 0));

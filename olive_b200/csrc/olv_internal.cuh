@@ -31,20 +31,22 @@ int cuda_fail(cudaError_t e, const char *what, const char *file, int line);
 // -------------------------------------------------------- device buffer --
 // A plain owned device allocation (no host mirror: the reference's GRD<T>,
 // grd.h:43-170, kept a host copy and synchronised it every superstep).
-// Freed when it goes out of scope; not copyable (a copy would free twice).
+// Given up when it goes out of scope, to be kept for the next buffer within a
+// bound (devmem.cu); not copyable (a copy would give it up twice).
 struct DevBuf {
     void *p = nullptr;
-    size_t bytes = 0;
+    size_t bytes = 0;         // what p has room for
+    int dev = 0;
     DevBuf() = default;
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
-    DevBuf(DevBuf &&o) noexcept : p(o.p), bytes(o.bytes) {
+    DevBuf(DevBuf &&o) noexcept : p(o.p), bytes(o.bytes), dev(o.dev) {
         o.p = nullptr;
         o.bytes = 0;
     }
     ~DevBuf() { release(); }
     int ensure(size_t n);     // grow to at least n bytes (contents not kept)
-    void release();
+    void release();           // waits for the device, as freeing does
     template <class T> T *as() const { return static_cast<T *>(p); }
 };
 
