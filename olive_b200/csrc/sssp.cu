@@ -860,7 +860,7 @@ __device__ void sssp_end_step(TravCtl *c, cudaGraphConditionalHandle h, int use_
 // handed back, so a run can change over at any superstep.
 // What bounds it: dependent L2 round trips of one SM (about 4 us a superstep of
 // 1300 edges).  Measured: 301 x 517 grid, weights U[1,255], 815 supersteps
-// 13.9 -> 3.3 ms; RMAT-24 1.69 -> 1.66 ms (its last supersteps; also the
+// 13.9 -> 3.3 ms; RMAT-24 1.69 -> 1.67 ms (its last supersteps; also the
 // distances and marks cleared by one launch).
 constexpr uint32_t kSmallFar = 16384;
 constexpr uint32_t kSmallHash = 1024;
@@ -878,7 +878,7 @@ struct SsspSmall {
 
 struct SmallShared {
     TravCtl c;
-    uint32_t vin[kSmallCap];                   // the superstep's input
+    uint32_t din[kSmallCap];                   // the superstep's input: distances
     SmallIndex ix;                             // its edges
     uint32_t v[kSmallCap], obeg[kSmallCap];    // the next one's
     uint16_t odeg[kSmallCap];                  // (at most kSmallEdges + 1: too many either way)
@@ -928,7 +928,7 @@ __device__ __forceinline__ void small_edges(const SsspSmall &x, const SmallStep 
                                             uint32_t total, uint32_t *dist, uint32_t &fmin,
                                             SmallShared &sh) {
     // each stage issues all its loads or atomics before any result is used
-    uint32_t at[N], src[N], du[N], old[N], nd[N], pos[N];
+    uint32_t at[N], du[N], old[N], nd[N], pos[N];
     uint2 e[N], r[N];
     bool act[N], near[N], far[N];
 #pragma unroll
@@ -936,18 +936,15 @@ __device__ __forceinline__ void small_edges(const SsspSmall &x, const SmallStep 
         const uint32_t k = base + j * kSmallThreads + threadIdx.x;
         act[j] = k < total;
         at[j] = 0;
-        src[j] = 0;
+        du[j] = 0;
         if (act[j]) {
             const uint32_t lo = sh.ix.owner(k);
             at[j] = sh.ix.beg[lo] + (k - sh.ix.off[lo]);
-            src[j] = sh.vin[lo];
+            du[j] = sh.din[lo];
         }
     }
 #pragma unroll
-    for (int j = 0; j < N; j++) {
-        e[j] = act[j] ? __ldg(&x.cw[at[j]]) : make_uint2(0u, 0u);
-        du[j] = act[j] ? __ldcg(&dist[src[j]]) : 0u;
-    }
+    for (int j = 0; j < N; j++) e[j] = act[j] ? __ldg(&x.cw[at[j]]) : make_uint2(0u, 0u);
 #pragma unroll
     for (int j = 0; j < N; j++) {
         nd[j] = du[j] + e[j].y;
@@ -1008,6 +1005,11 @@ __device__ bool small_relax(const SsspSmall &x, uint32_t n, uint32_t *dist, Smal
     unsigned long long relaxed = 0;
     bool drained = false;
     for (;;) {
+        // the input's distances, while its edges are numbered: one load a vertex, not
+        // one an edge (a vertex lowered meanwhile is queued again)
+        static_assert(kSmallCap == 2 * kSmallThreads, "two input vertices per thread");
+        const uint32_t d0 = t < n ? __ldcg(&dist[sh.v[t]]) : 0u;
+        const uint32_t d1 = t + kSmallThreads < n ? __ldcg(&dist[sh.v[t + kSmallThreads]]) : 0u;
         const uint32_t total = sh.ix.number(
             n, steps, [&](uint32_t i) { return (uint32_t)sh.odeg[i]; },
             [&](uint32_t i) { return sh.obeg[i]; });
@@ -1015,7 +1017,7 @@ __device__ bool small_relax(const SsspSmall &x, uint32_t n, uint32_t *dist, Smal
         // the bucket list, under the end step's capacity test
         const bool list = !a.all && !bl_over && (uint64_t)bl_size + n <= x.bl_cap;
         for (uint32_t i = t; i < n; i += kSmallThreads) {
-            sh.vin[i] = sh.v[i];
+            sh.din[i] = i < kSmallThreads ? d0 : d1;
             if (list) x.blist[bl_size + i] = sh.v[i];
         }
         sh.seen[t] = 0xffffffffu;
