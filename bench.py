@@ -465,17 +465,22 @@ def traversal_line(a, rank, world, local_rank, extra_keys=True):
     if traffic:
         roofline["traffic_over_algorithmic"] = round(traffic / alg_bytes, 3)
 
-    # launches of our kernels per step (kernel nodes executed by the graph):
+    # launches of our kernels per step (kernel nodes executed by the graph).
+    # Supersteps of small frontiers run inside the kernel that begins the run or
+    # ends a superstep, so for sssp and bfs the count is a lower bound: the
+    # supersteps that pulled are certain to have run the whole chain.
     # sssp: fill, init, 4 per superstep, the map back to the caller's ids
-    # (renumbered run), reached count; bfs: fill, init, 9 per level
+    # (renumbered run), reached count; bfs: fill, init, 7 per level; msbfs:
+    # init, 5 per level, levels; pagerank: init, control, 3 per iteration, map
+    # back, or init, one solve kernel, map back
     if a.workload == "sssp":
-        per_step = 2 + 4 * st.iterations + 1 + int(g.tune().get("sssp_relabel", 0))
+        per_step = 2 + 4 * st.pull_steps + 1 + int(g.tune().get("sssp_relabel", 0))
     elif a.workload == "bfs":
-        per_step = 2 + 9 * st.iterations
+        per_step = 2 + 7 * st.pull_steps
     elif a.workload == "msbfs":
-        per_step = 2 + 6 * st.iterations + 1
-    else:   # pagerank: segments (when the graph has long rows), blocks, fold per iteration
-        per_step = 2 + 3 * st.iterations
+        per_step = 2 + 5 * st.iterations
+    else:
+        per_step = 3 if E < 3 << 20 else 3 + 3 * st.iterations
     launches = per_step * a.steps
 
     # end to end through the public API: host (pinned) output buffer, D2H inside
@@ -735,7 +740,9 @@ def wpr_line(a, rank, world, local_rank):
         cpu = {"value": round(E * 3 / secs / 1e9, 5), "unit": "GE/s/iter", "cores": 1,
                "kind": "port", "sample": f"FP64 weighted PageRank forward (oracle), 3 sweeps, "
                                          f"{secs:.2f} s"}
-    launches = (2 + 3 * it) + (5 + 3 * it)
+    # forward: weights into both plans, out-weights, init, one solve, map back;
+    # backward: init, one solve, the transposed sums, the edge gradient
+    launches = 6 + 4
     config = workload_config(a, V, E, None, {
         "weights": "lognormal(0,1) FP32, numpy seed 7", "p": "Dirichlet(1)", "g": "N(0,1)",
         "alpha": 0.85, "sweeps": it, "forward_ms": round(ms_f, 3), "backward_ms": round(ms_b, 3)})
@@ -897,10 +904,13 @@ def ppr_line(a, rank, world, local_rank):
                 "kernel": "olv_ppr_batch solve (pull SpMM over the reverse graph, CUDA graph)",
                 "algorithmic_bytes": int(alg),
                 "bytes_formula": "per iteration: (4 B in-edge id + 4K B contribution row) per "
-                                 "edge + (x read, x write, y write: 12K B + 8 B) per vertex",
+                                 "edge + (x read, x write, y write: 12K B + 8 B) per vertex; counts "
+                                 "every row gather, rows gathered again come from L2",
                 "peak_source": peak_src, "kernel_ms": round(kern_ms, 4)}
     traffic, traffic_src = profile_traffic("ppr", a.scale, a.seed)
     roofline.update(traffic=traffic, traffic_source=traffic_src)
+    if traffic:
+        roofline["dram_frac"] = round(traffic / (kern_ms * 1e-3) / 1e9 / peak, 4)
     host = torch.empty((V, K), dtype=torch.float32, pin_memory=True)
     t0 = time.perf_counter()
     for _ in range(a.steps):
@@ -924,7 +934,7 @@ def ppr_line(a, rank, world, local_rank):
     config["workload"] = f"ppr32-rmat{a.scale}"
     line = common_line(a, world, "GE/s/iter", value, ms, "f32",
                        "synthetic (seeded RMAT, generated on the device)", config, roofline,
-                       None, e2e, a.steps * (3 * it + 4), clk, extra)
+                       None, e2e, a.steps * (3 * it + 3), clk, extra)
     g.close()
     return line
 

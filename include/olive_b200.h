@@ -146,6 +146,7 @@ int olv_graph_max_degree_vertex(const olv_graph *g, uint32_t *v, uint32_t *deg);
  *                 the lanes per row of the tile plans, rebuilt on change;
  *                 a weighted-PR backward needs its forward run after it (8)
  *   "use_graphs"  run supersteps inside CUDA graphs (1) or a host loop (0)
+ *                 (solves that run in one launch, as weighted PageRank's, ignore it)
  *   "levels_per_sync" host loop: supersteps enqueued per check      (4)
  *   "batch_cluster" olv_batch_run: PPR items on thread-block clusters of
  *                 8 or 16 CTAs (1 = the largest the GPU runs), or one CTA per
