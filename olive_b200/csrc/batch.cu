@@ -718,6 +718,7 @@ extern "C" int olv_batch_run(olv_graph *g, const uint32_t *inst_offsets, int cou
                              int32_t *levels_out, float *ppr_out, uint32_t *ppr_iters_out,
                              olv_stats *st) {
     OLV_CHECK_ARG(g && inst_offsets, "olv_batch_run: null pointer");
+    BufferScope scope(g->stream);
     OLV_CHECK_ARG(count >= 1, "olv_batch_run: count must be >= 1");
     OLV_CHECK_ARG(levels_out || ppr_out, "olv_batch_run: nothing to compute");
     OLV_CHECK_ARG(!ppr_out || (seeds && K >= 1 && K <= 32),

@@ -939,6 +939,7 @@ using namespace olv;
 
 extern "C" int olv_bfs(olv_graph *g, uint32_t src, int32_t *level_out, olv_stats *st) {
     OLV_CHECK_ARG(g && level_out, "olv_bfs: null pointer");
+    BufferScope scope(g->stream);
     OLV_CHECK_ARG(src < g->V, "olv_bfs: source %u out of range (V=%u)", src, g->V);
     OLV_TRY(traversal_workspace(g, true));
     OLV_TRY(bfs_pull_lists(g));

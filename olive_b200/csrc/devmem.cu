@@ -15,9 +15,12 @@
 //   - when the driver has no room for a new buffer, every kept block of the
 //     device goes back and the allocation is tried again, so that keeping
 //     blocks never makes one of the engine's allocations fail;
-//   - a block is kept only after the device has finished all work submitted so
-//     far (what freeing it waits for as well), so its next owner may use it on
-//     any stream and from any thread; the lists are guarded by one mutex.
+//   - a block is kept only by a call on a handle (BufferScope), after the
+//     handle's stream, the only one that uses the handle's buffers, has been
+//     waited for, so its next owner may use it on any stream and from any
+//     thread; no other stream is waited for or looked at, so captures that
+//     other threads have under way are not disturbed.  What is given up
+//     elsewhere is freed.  The lists are guarded by one mutex.
 #include <list>
 #include <mutex>
 #include <unordered_map>
@@ -104,13 +107,16 @@ cudaError_t take(Block *out, size_t n) {
     return cudaSuccess;
 }
 
+// The scope this thread is in.
+thread_local cudaStream_t t_stream = nullptr;
+thread_local bool t_keep = false;
+
 void put(const Block &b) {
     int dev = 0;
-    bool idle = cudaGetDevice(&dev) == cudaSuccess;
-    if (idle && dev != b.dev) idle = cudaSetDevice(b.dev) == cudaSuccess;
-    idle = idle && cudaDeviceSynchronize() == cudaSuccess;
-    bool keep = false;
-    if (idle) {
+    bool keep = t_keep && cudaGetDevice(&dev) == cudaSuccess && dev == b.dev &&
+                cudaStreamSynchronize(t_stream) == cudaSuccess;
+    if (keep) {
+        keep = false;
         Kept &k = kept();
         std::lock_guard<std::mutex> lock(k.m);
         try {
@@ -125,10 +131,19 @@ void put(const Block &b) {
         }
     }
     if (!keep) cudaFree(b.p);
-    if (dev != b.dev) cudaSetDevice(dev);
 }
 
 }  // namespace
+
+BufferScope::BufferScope(cudaStream_t s, bool keep) : before(t_stream), kept_before(t_keep) {
+    t_stream = s;
+    t_keep = keep;
+}
+
+BufferScope::~BufferScope() {
+    t_stream = before;
+    t_keep = kept_before;
+}
 
 int DevBuf::ensure(size_t n) {
     if (n <= bytes && p) return OLV_OK;

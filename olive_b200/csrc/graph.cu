@@ -319,6 +319,7 @@ int olv_graph_create(const uint32_t *rowptr, const uint32_t *col, const void *we
     *out = nullptr;
     olv_graph *g = nullptr;
     OLV_TRY(new_graph(&g));
+    BufferScope scope(g->stream);
     g->V = V;
     g->E = E;
     g->weight_type = weight_type;
@@ -353,6 +354,7 @@ int olv_graph_create_rmat(int scale, int edge_factor, uint64_t seed, int weight_
     *out = nullptr;
     olv_graph *g = nullptr;
     OLV_TRY(new_graph(&g));
+    BufferScope scope(g->stream);
     g->V = (uint32_t)V;
     g->weight_type = weight_type;
     cudaStream_t s = g->stream;
@@ -432,6 +434,7 @@ int olv_graph_destroy(olv_graph *g) {
     if (!g) return OLV_OK;
     cudaSetDevice(g->device);
     if (g->stream) cudaStreamSynchronize(g->stream);
+    BufferScope scope(g->stream);
     g->rowptr.release(); g->col.release(); g->w.release();
     g->colptr.release(); g->rowidx.release(); g->csc_w.release(); g->csc_eid.release();
     g->outdeg_f.release();
@@ -451,6 +454,7 @@ int olv_graph_destroy(olv_graph *g) {
     if (g->host_ctl) cudaFreeHost(g->host_ctl);
     if (g->ev0) cudaEventDestroy(g->ev0);
     if (g->ev1) cudaEventDestroy(g->ev1);
+    BufferScope none(nullptr, false);   // the stream goes
     if (g->own_stream) cudaStreamDestroy(g->own_stream);
     delete g;
     return OLV_OK;

@@ -735,6 +735,7 @@ using namespace olv;
 extern "C" int olv_msbfs(olv_graph *g, const uint32_t *srcs, int n, int32_t *levels_out,
                          olv_stats *st) {
     OLV_CHECK_ARG(g && srcs && levels_out, "olv_msbfs: null pointer");
+    BufferScope scope(g->stream);
     OLV_CHECK_ARG(n >= 1 && n <= 64, "olv_msbfs: n=%d sources, must be in [1,64]", n);
     const bool dev_src = is_device_ptr(srcs);
     std::vector<uint32_t> hs(n);

@@ -46,8 +46,22 @@ struct DevBuf {
     }
     ~DevBuf() { release(); }
     int ensure(size_t n);     // grow to at least n bytes (contents not kept)
-    void release();           // waits for the device, as freeing does
+    void release();           // keeps it for the next buffer (BufferScope) or frees it
     template <class T> T *as() const { return static_cast<T *>(p); }
+};
+
+// While one stands, buffers that this thread gives up are kept for the next ones
+// once `s`, the only stream that uses them, is idle; otherwise they are freed.
+class BufferScope {
+public:
+    explicit BufferScope(cudaStream_t s, bool keep = true);
+    ~BufferScope();
+    BufferScope(const BufferScope &) = delete;
+    BufferScope &operator=(const BufferScope &) = delete;
+
+private:
+    cudaStream_t before;
+    bool kept_before;
 };
 
 // Where a caller's pointer lives.

@@ -326,6 +326,7 @@ void olv::release_pr_state(olv_graph *g) {
 extern "C" int olv_pagerank(olv_graph *g, double alpha, int max_it, double tol, int dangling_mode,
                             float *rank_out, olv_stats *st) {
     OLV_CHECK_ARG(g && rank_out, "olv_pagerank: null pointer");
+    BufferScope scope(g->stream);
     OLV_CHECK_ARG(alpha >= 0.0 && alpha < 1.0, "olv_pagerank: alpha must be in [0,1)");
     OLV_CHECK_ARG(max_it >= 0, "olv_pagerank: max_it must be >= 0");
     OLV_CHECK_ARG(dangling_mode == OLV_DANGLING_UNIFORM || dangling_mode == OLV_DANGLING_LEAK,

@@ -569,6 +569,7 @@ void olv::release_ppr_state(olv_graph *g) {
 extern "C" int olv_ppr_batch(olv_graph *g, const uint32_t *seeds, int K, double alpha,
                              int max_it, double tol, float *out, olv_stats *st) {
     OLV_CHECK_ARG(g && seeds && out, "olv_ppr_batch: null pointer");
+    BufferScope scope(g->stream);
     OLV_CHECK_ARG(K >= 1 && K <= kPprK, "olv_ppr_batch: K must be in [1, %d]", kPprK);
     OLV_CHECK_ARG(alpha >= 0.0 && alpha < 1.0, "olv_ppr_batch: alpha must be in [0,1)");
     OLV_CHECK_ARG(max_it >= 0, "olv_ppr_batch: max_it must be >= 0");

@@ -1734,6 +1734,7 @@ using namespace olv;
 
 extern "C" int olv_sssp(olv_graph *g, uint32_t src, uint32_t *dist_out, olv_stats *st) {
     OLV_CHECK_ARG(g && dist_out, "olv_sssp: null pointer");
+    BufferScope scope(g->stream);
     OLV_CHECK_ARG(src < g->V, "olv_sssp: source %u out of range (V=%u)", src, g->V);
     OLV_CHECK_ARG(g->weight_type == OLV_W_U32, "olv_sssp: graph has no uint32 weights");
     OLV_TRY(sssp_workspace(g));

@@ -313,6 +313,7 @@ extern "C" int olv_wpr_forward(olv_graph *g, const float *w, const float *p, dou
                                int max_it, double tol, float *r_out, olv_wpr_ctx **ctx_out,
                                olv_stats *st) {
     OLV_CHECK_ARG(g && p && ctx_out, "olv_wpr_forward: null pointer");
+    BufferScope scope(g->stream);
     OLV_CHECK_ARG(alpha >= 0 && alpha < 1 && max_it >= 0, "olv_wpr_forward: bad alpha / max_it");
     if (w) OLV_TRY(olv_graph_set_weights_f32(g, w));
     OLV_CHECK_ARG(g->weight_type == OLV_W_F32, "olv_wpr_forward: graph has no FP32 weights");
@@ -394,6 +395,7 @@ extern "C" int olv_wpr_backward(olv_wpr_ctx *c, const float *gvec, int max_it, d
     OLV_CHECK_ARG(c && c->g && gvec && dw_out, "olv_wpr_backward: null pointer or no forward");
     OLV_CHECK_ARG(max_it >= 0, "olv_wpr_backward: bad max_it");
     olv_graph *g = c->g;
+    BufferScope scope(g->stream);
     if (!wpr_plans(g)) {   // the row plans were dropped (pr_tile_u changed) since the forward
         set_error("olv_wpr_backward: the graph's row plans changed since olv_wpr_forward; "
                   "run the forward again");
