@@ -484,6 +484,8 @@ int olv_graph_copy_csr(const olv_graph *g, uint32_t *rowptr, uint32_t *col, void
 int olv_graph_set_weights_f32(olv_graph *g, const float *w) {
     OLV_CHECK_ARG(g && (w || g->E == 0), "olv_graph_set_weights_f32: null pointer");
     OLV_TRY(copy_in(g->w, w, g->E * 4, g->stream));
+    // the handle may be moved to another stream next, which would not wait for this
+    OLV_CUDA(cudaStreamSynchronize(g->stream));
     // no CSC copy: only SSSP reads one, and its weights are uint32
     g->weight_type = OLV_W_F32;
     return OLV_OK;
