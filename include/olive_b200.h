@@ -102,6 +102,12 @@ int olv_graph_copy_csr(const olv_graph *g, uint32_t *rowptr, uint32_t *col, void
 int olv_graph_set_weights_f32(olv_graph *g, const float *w);
 /* Bind the handle to a CUDA stream (a cudaStream_t; NULL = the handle's own). */
 int olv_set_stream(olv_graph *g, void *stream);
+/* Device memory that handles gave up is kept for the next buffers, at most 1/64
+ * of the device's memory (no reference counterpart).  This call gives what is
+ * kept in the calling thread's context back to the driver, for the other users
+ * of the device; *bytes_out (if not NULL) gets the bytes.  The engine does the
+ * same when one of its own allocations finds no room.                         */
+int olv_release_memory(uint64_t *bytes_out);
 /* Maximum out-degree vertex, ties to the smallest id. */
 int olv_graph_max_degree_vertex(const olv_graph *g, uint32_t *v, uint32_t *deg);
 /* Engine tunables by name (no reference counterpart; the reference fixed its

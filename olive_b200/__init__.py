@@ -11,7 +11,8 @@ import os
 
 import numpy as np
 
-__all__ = ["Graph", "OliveError", "lib", "INF", "Stats", "write_csr_binary", "write_text"]
+__all__ = ["Graph", "OliveError", "lib", "INF", "Stats", "release_memory", "write_csr_binary",
+           "write_text"]
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libolive_b200.so")
@@ -85,6 +86,7 @@ _SIGS = [
     ("olv_graph_copy_csr", _I, [_VP, _VP, _VP, _VP]),
     ("olv_graph_set_weights_f32", _I, [_VP, _VP]),
     ("olv_set_stream", _I, [_VP, _VP]),
+    ("olv_release_memory", _I, [ctypes.POINTER(_U64)]),
     ("olv_graph_max_degree_vertex", _I, [_VP, ctypes.POINTER(_U32), ctypes.POINTER(_U32)]),
     ("olv_tune_set", _I, [_VP, ctypes.c_char_p, _D]),
     ("olv_tune_get", _I, [_VP, ctypes.c_char_p, ctypes.POINTER(_D)]),
@@ -158,6 +160,14 @@ def _u32(a):
         import torch
         return a.to(torch.int32).contiguous() if a.dtype != torch.int32 else a.contiguous()
     return np.ascontiguousarray(a, dtype=np.uint32)
+
+
+def release_memory():
+    """Give the device memory kept from closed graphs back to the driver
+    (olv_release_memory), as before a large allocation elsewhere.  Returns the bytes."""
+    out = _U64()
+    _check(lib().olv_release_memory(ctypes.byref(out)), "olv_release_memory")
+    return out.value
 
 
 class Graph:

@@ -9,21 +9,27 @@
 // quarter of itself.
 //
 // Bounds and safety:
-//   - at most 1/64 of a device's memory is kept on it; past that the blocks
-//     kept longest go back to the driver first, and a block larger than the
-//     bound goes back at once;
+//   - at most 1/64 of a device's memory is kept in a context; past that the
+//     blocks kept longest go back to the driver first (cudaFree, which may wait
+//     for the device), and a block larger than the bound goes back at once;
 //   - when the driver has no room for a new buffer, every kept block of the
-//     device goes back and the allocation is tried again, so that keeping
-//     blocks never makes one of the engine's allocations fail;
+//     context goes back and the allocation is tried again, so that keeping
+//     blocks never makes one of the engine's allocations fail; other users of the
+//     device get them with olv_release_memory();
 //   - a block is kept only by a call on a handle (BufferScope), after the
 //     handle's stream, the only one that uses the handle's buffers, has been
 //     waited for, so its next owner may use it on any stream and from any
-//     thread; no other stream is waited for or looked at, so captures that
-//     other threads have under way are not disturbed.  What is given up
-//     elsewhere is freed.  The lists are guarded by one mutex.
+//     thread.  Keeping a block and handing it out again wait for no other
+//     stream.  What is given up elsewhere is freed.  The lists are guarded by one
+//     mutex;
+//   - a block belongs to the context it was allocated in and is handed out there
+//     only: a context's id is never used again, so that blocks which died with
+//     their context (cudaDeviceReset, cuCtxDestroy) stay where they are.
 #include <list>
 #include <mutex>
 #include <unordered_map>
+
+#include <cudaTypedefs.h>
 
 #include "olv_internal.cuh"
 
@@ -36,14 +42,17 @@ constexpr size_t kSmallUnit = 512, kLargeUnit = 2u << 20;   // block sizes are m
 struct Block {
     void *p;
     size_t bytes;
-    int dev;
+    uint64_t ctx;
+};
+
+struct PerContext {
+    size_t bytes = 0, bound = 0;
 };
 
 struct Kept {
     std::mutex m;
-    std::list<Block> blocks;                    // kept longest first
-    std::unordered_map<int, size_t> bytes;      // kept, by device
-    std::unordered_map<int, size_t> bound;
+    std::list<Block> blocks;   // kept longest first
+    std::unordered_map<uint64_t, PerContext> by_ctx;
 };
 
 Kept &kept() {
@@ -51,27 +60,56 @@ Kept &kept() {
     return *k;
 }
 
-size_t keep_bound(Kept &k, int dev) {
-    auto it = k.bound.find(dev);
-    if (it != k.bound.end()) return it->second;
+template <class Fn>
+Fn driver_entry(const char *name) {
+    void *fn = nullptr;
+    cudaDriverEntryPointQueryResult found;
+    if (cudaGetDriverEntryPointByVersion(name, &fn, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return reinterpret_cast<Fn>(fn);
+}
+
+// Id of the calling thread's context, 0 if it cannot be told (nothing is kept then).
+uint64_t current_context() {
+    static const auto get = driver_entry<PFN_cuCtxGetCurrent_v4000>("cuCtxGetCurrent");
+    static const auto id_of = driver_entry<PFN_cuCtxGetId_v12000>("cuCtxGetId");
+    if (!get || !id_of) return 0;
+    CUcontext c = nullptr;
+    if (get(&c) != CUDA_SUCCESS || !c) {
+        // this thread's first call: the runtime has not made a context current yet
+        if (cudaFree(nullptr) != cudaSuccess || get(&c) != CUDA_SUCCESS || !c) {
+            cudaGetLastError();
+            return 0;
+        }
+    }
+    unsigned long long id = 0;
+    return id_of(c, &id) == CUDA_SUCCESS ? id : 0;
+}
+
+size_t keep_bound() {
     size_t free_b = 0, total = 0;
     if (cudaMemGetInfo(&free_b, &total) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }
-    return k.bound[dev] = total / 64;
+    return total / 64;
 }
 
-// Blocks of device dev, kept longest first, go back to the driver until at
-// most `most` bytes are kept there.
-void give_back(Kept &k, int dev, size_t most) {
-    for (auto it = k.blocks.begin(); it != k.blocks.end() && k.bytes[dev] > most;) {
-        if (it->dev != dev) {
+// Blocks of the current context ctx, kept longest first, go back to the driver
+// until at most `most` bytes are kept there.
+void give_back(Kept &k, uint64_t ctx, size_t most) {
+    const auto c = k.by_ctx.find(ctx);
+    if (c == k.by_ctx.end()) return;
+    for (auto it = k.blocks.begin(); it != k.blocks.end() && c->second.bytes > most;) {
+        if (it->ctx != ctx) {
             ++it;
             continue;
         }
         cudaFree(it->p);
-        k.bytes[dev] -= it->bytes;
+        c->second.bytes -= it->bytes;
         it = k.blocks.erase(it);
     }
 }
@@ -79,26 +117,24 @@ void give_back(Kept &k, int dev, size_t most) {
 cudaError_t take(Block *out, size_t n) {
     const size_t unit = n < kLargeUnit / 2 ? kSmallUnit : kLargeUnit;
     const size_t need = (n + unit - 1) / unit * unit;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
+    const uint64_t ctx = current_context();
     Kept &k = kept();
     std::lock_guard<std::mutex> lock(k.m);
     auto best = k.blocks.end();
     for (auto it = k.blocks.begin(); it != k.blocks.end(); ++it)
-        if (it->dev == dev && it->bytes >= need && it->bytes - need <= it->bytes / 4 &&
+        if (it->ctx == ctx && it->bytes >= need && it->bytes - need <= it->bytes / 4 &&
             (best == k.blocks.end() || it->bytes < best->bytes))
             best = it;
-    Block b{nullptr, need, dev};
+    Block b{nullptr, need, ctx};
     if (best != k.blocks.end()) {
         b = *best;
-        k.bytes[dev] -= b.bytes;
+        k.by_ctx.find(ctx)->second.bytes -= b.bytes;
         k.blocks.erase(best);
     } else {
-        e = cudaMalloc(&b.p, need);
-        if (e == cudaErrorMemoryAllocation && k.bytes[dev]) {
+        cudaError_t e = cudaMalloc(&b.p, need);
+        if (e == cudaErrorMemoryAllocation) {
             cudaGetLastError();
-            give_back(k, dev, 0);
+            give_back(k, ctx, 0);
             e = cudaMalloc(&b.p, need);
         }
         if (e != cudaSuccess) return e;
@@ -112,19 +148,19 @@ thread_local cudaStream_t t_stream = nullptr;
 thread_local bool t_keep = false;
 
 void put(const Block &b) {
-    int dev = 0;
-    bool keep = t_keep && cudaGetDevice(&dev) == cudaSuccess && dev == b.dev &&
+    bool keep = t_keep && b.ctx && current_context() == b.ctx &&
                 cudaStreamSynchronize(t_stream) == cudaSuccess;
     if (keep) {
         keep = false;
         Kept &k = kept();
         std::lock_guard<std::mutex> lock(k.m);
         try {
-            const size_t bound = keep_bound(k, b.dev);
-            if (b.bytes <= bound) {
-                give_back(k, b.dev, bound - b.bytes);
+            PerContext &c = k.by_ctx[b.ctx];
+            if (c.bound == 0) c.bound = keep_bound();
+            if (b.bytes <= c.bound) {
+                give_back(k, b.ctx, c.bound - b.bytes);
                 k.blocks.push_back(b);
-                k.bytes[b.dev] += b.bytes;
+                c.bytes += b.bytes;
                 keep = true;
             }
         } catch (...) {   // no host memory for the list: not kept
@@ -154,14 +190,26 @@ int DevBuf::ensure(size_t n) {
     if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc", __FILE__, __LINE__);
     p = b.p;
     bytes = b.bytes;
-    dev = b.dev;
+    ctx = b.ctx;
     return OLV_OK;
 }
 
 void DevBuf::release() {
-    if (p) put(Block{p, bytes, dev});
+    if (p) put(Block{p, bytes, ctx});
     p = nullptr;
     bytes = 0;
 }
 
 }  // namespace olv
+
+using namespace olv;
+
+extern "C" int olv_release_memory(uint64_t *bytes_out) {
+    const uint64_t ctx = current_context();
+    Kept &k = kept();
+    std::lock_guard<std::mutex> lock(k.m);
+    const auto c = k.by_ctx.find(ctx);
+    if (bytes_out) *bytes_out = c == k.by_ctx.end() ? 0 : c->second.bytes;
+    give_back(k, ctx, 0);
+    return OLV_OK;
+}

@@ -36,11 +36,11 @@ int cuda_fail(cudaError_t e, const char *what, const char *file, int line);
 struct DevBuf {
     void *p = nullptr;
     size_t bytes = 0;         // what p has room for
-    int dev = 0;
+    uint64_t ctx = 0;         // id of the context p belongs to
     DevBuf() = default;
     DevBuf(const DevBuf &) = delete;
     DevBuf &operator=(const DevBuf &) = delete;
-    DevBuf(DevBuf &&o) noexcept : p(o.p), bytes(o.bytes), dev(o.dev) {
+    DevBuf(DevBuf &&o) noexcept : p(o.p), bytes(o.bytes), ctx(o.ctx) {
         o.p = nullptr;
         o.bytes = 0;
     }
