@@ -744,7 +744,7 @@ __global__ void k_first_parent(const uint32_t *__restrict__ colptr,
 // (the ones a BFS reaches first); built once per graph.
 int bfs_pull_lists(olv_graph *g) {
     Workspace &w = g->ws;
-    if (w.order.p) return OLV_OK;
+    if (w.pull_built) return OLV_OK;   // all of them: an allocation below may have failed before
     const uint32_t V = g->V;
     cudaStream_t s = g->stream;
     DevBuf key, val, key2, temp, cnt;
@@ -803,6 +803,7 @@ int bfs_pull_lists(olv_graph *g) {
                                                     w.pull_first.as<uint32_t>());
     OLV_CUDA(cudaGetLastError());
     OLV_CUDA(cudaStreamSynchronize(s));
+    w.pull_built = 1;
     return OLV_OK;
 }
 

@@ -102,6 +102,7 @@ struct Workspace {
     DevBuf order, cand, cand2;      // BFS pull: in-degree-sorted vertices, candidate lists
     DevBuf pull_first;              // BFS pull: each vertex's first in-edge in pull order
     DevBuf pull_idx;                // BFS pull: in-edges sorted by source out-degree (desc)
+    int pull_built = 0;             // BFS pull: the five above are complete
     // SSSP: rows split light (w <= delta) | heavy, as (column, weight) pairs;
     // rowmid[u] the split point; per vertex its light and heavy ranges as
     // uint2 (one load each); the in-edges as (source, weight) pairs
@@ -123,6 +124,7 @@ struct Workspace {
         level.release(); q0.release(); q1.release(); pieces.release(); ctl.release();
         fbits.release(); order.release(); cand.release(); cand2.release(); pull_idx.release();
         pull_first.release();
+        pull_built = 0;
         sssp_cw.release(); rowmid.release(); sssp_lr.release(); sssp_hr.release();
         sssp_crw.release(); blist.release(); hdin.release();
         sssp_delta_built = 0;
