@@ -546,12 +546,8 @@ k_row_solve(SolveArgs a, Op op) {
     }
 }
 
-// Whether the GPU runs a cluster of kClusterCTAs CTAs of 217 KB.
-template <class Op>
-bool cluster_fits(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr, const SolvePlan &p,
-                  cudaStream_t s) {
-    const void *fn = (const void *)k_row_solve<Op, true>;
-    const size_t smem = Op::kGather ? ((size_t)p.n + 4) * 4 : 0;
+inline void cluster_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr, size_t smem,
+                           cudaStream_t s) {
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = kClusterCTAs;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
@@ -562,14 +558,32 @@ bool cluster_fits(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr, const Solv
     cfg->stream = s;
     cfg->attrs = attr;
     cfg->numAttrs = 1;
+}
+
+// Whether the GPU runs the cluster form of Op at its largest.  The attributes belong
+// to the kernel, whatever handle or thread launches it, so they are set to the most
+// that any plan needs and never lowered.
+template <class Op>
+bool cluster_runs() {
+    const void *fn = (const void *)k_row_solve<Op, true>;
+    const int smem = Op::kGather ? (int)((kClusterRows + 4) * 4) : 0;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[1];
+    cluster_config(&cfg, attr, (size_t)smem, nullptr);
     int n = 0;
     const bool ok =
         cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) ==
-            cudaSuccess &&
-        cudaOccupancyMaxActiveClusters(&n, fn, cfg) == cudaSuccess && n >= 1;
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
+        cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess && n >= 1;
     if (!ok) cudaGetLastError();
     return ok;
+}
+
+// The form a plan's solves take, decided once, when it is built: a cluster where the
+// plan is small and the GPU runs one for every Op it is used with.
+template <class... Ops>
+void choose_form(SolvePlan &p) {
+    if (p.cluster) p.cluster = (cluster_runs<Ops>() && ...);
 }
 
 // Launch a solve.  *ctl must be zero but for count.
@@ -578,10 +592,9 @@ int launch_solve(const SolvePlan &p, SolveArgs a, Op op, cudaStream_t s) {
     if (p.cluster) {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr[1];
-        if (cluster_fits<Op>(&cfg, attr, p, s)) {
-            OLV_CUDA(cudaLaunchKernelEx(&cfg, k_row_solve<Op, true>, a, op));
-            return OLV_OK;
-        }
+        cluster_config(&cfg, attr, Op::kGather ? ((size_t)p.n + 4) * 4 : 0, s);
+        OLV_CUDA(cudaLaunchKernelEx(&cfg, k_row_solve<Op, true>, a, op));
+        return OLV_OK;
     }
     void *args[] = {&a, &op};
     OLV_CUDA(cudaLaunchCooperativeKernel((const void *)k_row_solve<Op, false>, dim3(p.grid),

@@ -261,12 +261,14 @@ struct PrPlan {
 static int build_pr_plan(olv_graph *g, PrPlan &p) {
     const uint32_t V = g->V;
     p.solve = g->E < kPrSolveEdges || g->max_in_degree <= kRowLong;
-    if (p.solve)
+    if (p.solve) {
         OLV_TRY(build_solve_plan(g->colptr.as<uint32_t>(), g->rowidx.as<uint32_t>(), nullptr, V,
                                  g->E, g->tune.pr_tile_u, false, g->num_sms, g->stream, p.sp));
-    else
+        choose_form<PrOp>(p.sp);
+    } else {
         OLV_TRY(build_tile_plan(g->colptr.as<uint32_t>(), g->rowidx.as<uint32_t>(), V, g->stream,
                                 p.tp, g->tune.pr_tile_u));
+    }
     OLV_TRY(p.outdeg.ensure((size_t)V * 4 + 16));
     k_outdeg_perm<<<g->num_sms * 8, kBlock, 0, g->stream>>>(g->rowptr.as<uint32_t>(), p.perm(), V,
                                                            p.outdeg.as<uint32_t>());

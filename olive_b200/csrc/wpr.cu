@@ -283,6 +283,8 @@ static int ensure_wpr_plans(olv_graph *g) {
         delete p;
         return r;
     }
+    choose_form<WfwdOp>(p->tcsc);
+    choose_form<WsumOp, WadjOp, WtOp>(p->tcsr);
     k_grad_rows<<<g->num_sms * 8, kBlock, 0, s>>>(g->rowptr.as<uint32_t>(), g->V, g->E,
                                                  p->erow.as<uint32_t>());
     g->wpr_state = p;
