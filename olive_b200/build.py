@@ -33,6 +33,7 @@ def nvcc():
 
 def _headers():
     return glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(
+        os.path.join(CSRC, "*.h")) + glob.glob(
         os.path.join(ROOT, "include", "*.h")) + glob.glob(
         os.path.join(ROOT, "include", "olive_b200", "*.cuh"))
 

@@ -29,8 +29,7 @@
 #include <mutex>
 #include <unordered_map>
 
-#include <cudaTypedefs.h>
-
+#include "olv_driver.h"
 #include "olv_internal.cuh"
 
 namespace olv {
@@ -60,22 +59,10 @@ Kept &kept() {
     return *k;
 }
 
-template <class Fn>
-Fn driver_entry(const char *name) {
-    void *fn = nullptr;
-    cudaDriverEntryPointQueryResult found;
-    if (cudaGetDriverEntryPointByVersion(name, &fn, 12000, cudaEnableDefault, &found) != cudaSuccess ||
-        found != cudaDriverEntryPointSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    return reinterpret_cast<Fn>(fn);
-}
-
 // Id of the calling thread's context, 0 if it cannot be told (nothing is kept then).
 uint64_t current_context() {
-    static const auto get = driver_entry<PFN_cuCtxGetCurrent_v4000>("cuCtxGetCurrent");
-    static const auto id_of = driver_entry<PFN_cuCtxGetId_v12000>("cuCtxGetId");
+    static const auto get = driver_entry<PFN_cuCtxGetCurrent_v4000>("cuCtxGetCurrent", 4000);
+    static const auto id_of = driver_entry<PFN_cuCtxGetId_v12000>("cuCtxGetId", 12000);
     if (!get || !id_of) return 0;
     CUcontext c = nullptr;
     if (get(&c) != CUDA_SUCCESS || !c) {

@@ -16,8 +16,8 @@
 // every CTA copies all gathered values to shared memory at the start of an
 // iteration (16 SMs read at most 217 KB each, contiguous), where 32 gathers take
 // 3-4 cycles of bank conflicts instead of 32 lookups in L1, and the barrier
-// between two iterations is the cluster's.  Larger ones take the whole GPU by a
-// cooperative launch: at the grid barrier the last CTA to arrive adds up the
+// between two iterations is the cluster's.  Larger ones take the whole GPU (join_team
+// below): at the grid barrier the last CTA to arrive adds up the
 // FP64 partials in a fixed order and takes the decision for all.  What bounds
 // those is the gathers: a 4-byte gather that misses L1 is a request of its own
 // to L2 and an SM sends one per cycle, so as many warps as possible keep eight
@@ -119,6 +119,8 @@ struct RowClassTable {
 };
 
 struct SolveCtl {
+    uint32_t joined;     // CTAs that came before the team was closed (then kTeamClosed is set)
+    uint32_t team;       // CTAs of the run, 0 until it is closed
     uint32_t arrive;     // barrier arrivals of the run
     uint32_t go;         // iterations whose barrier is open
     uint32_t err;        // a wait ran out
@@ -193,6 +195,9 @@ int build_solve_plan(const uint32_t *ptr, const uint32_t *idx, const uint32_t *e
                      uint64_t nnz, uint32_t lanes_u, bool with_pos, int num_sms, cudaStream_t s,
                      SolvePlan &p);
 
+// Whether the stream may use every SM (it does not belong to a green context).
+bool stream_has_whole_gpu(cudaStream_t s);
+
 inline int solve_error(const SolveCtl &c, const char *what) {
     if (!c.err) return OLV_OK;
     set_error("%s: a grid barrier ran out of time", what);
@@ -203,6 +208,45 @@ inline int solve_error(const SolveCtl &c, const char *what) {
 
 // Polls allowed in a grid barrier: seconds, far above any iteration.
 constexpr uint32_t kBarrierPolls = 1u << 25;
+
+// The CTAs that run a whole-GPU solve: those that are there when it starts.  A grid
+// barrier needs every CTA that waits at it to run at once, and on part of a GPU (a
+// green context, an MPS share) or beside another stream's kernels the launch may
+// not fit.  So a CTA joins by a counter; when all of the grid have joined, or
+// kJoinNs after the first, the team is closed, and a CTA that comes later leaves.
+// Every member was running when it joined, so the barriers end whatever runs
+// beside them.  The grid's shares of the work go to the members in turn and the sums
+// of a share have a place of their own, so results do not depend on the team.
+// A cooperative launch instead fails where the grid does not fit and waits until
+// all of it does.
+constexpr uint32_t kTeamClosed = 1u << 31;
+constexpr uint64_t kJoinNs = 100000;
+
+// One thread per CTA.  False: too late, or (err set) the wait ran out.
+__device__ __forceinline__ bool join_team(SolveCtl *ctl, uint32_t grid, uint32_t &rank,
+                                          uint32_t &team) {
+    rank = atomicAdd(&ctl->joined, 1u);
+    if (rank & kTeamClosed) return false;
+    auto close = [&] {
+        const uint32_t n = atomicOr(&ctl->joined, kTeamClosed);
+        if (!(n & kTeamClosed))
+            asm volatile("st.release.gpu.u32 [%0], %1;" ::"l"(&ctl->team), "r"(n) : "memory");
+    };
+    uint64_t start, now;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(start));
+    if (rank + 1 == grid) close();
+    for (uint32_t i = 0; i < kBarrierPolls; i++) {
+        asm volatile("ld.acquire.gpu.u32 %0, [%1];" : "=r"(team) : "l"(&ctl->team) : "memory");
+        if (team) return true;
+        if (rank == 0) {
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+            if (now - start >= kJoinNs) close();
+        }
+        if (i > 64) __nanosleep(64);
+    }
+    ctl->err = 1;
+    return false;
+}
 
 // Value of id j, 0 for a place without an entry (id none), by one predicated load:
 // no request for such a place, no branch, several in flight.
@@ -228,20 +272,32 @@ k_row_solve(SolveArgs a, Op op) {
     __shared__ double s_sum[2];
     __shared__ double s_part[2][2];   // kCluster: this CTA's sums, by iteration parity
     __shared__ uint32_t s_state;   // barrier: 0 out of time, 1 open, 2 this CTA is the last
+    __shared__ uint32_t s_rank, s_team;   // !kCluster: this CTA in its team, CTAs in it
     constexpr unsigned kFull = 0xffffffffu;
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const uint32_t gw = blockIdx.x * kWarps + wid, nw = gridDim.x * kWarps;
+    const uint32_t nw = gridDim.x * kWarps;
     const uint32_t ntiles = a.cls.tile0[kRowClasses], nfull = a.cls.tile0[kRowClasses - 1];
     const uint32_t nlong = a.cls.row0[1];
+    uint32_t rank = blockIdx.x;
+    if constexpr (!kCluster) {
+        if (threadIdx.x == 0) {
+            uint32_t r, n;
+            s_team = join_team(a.ctl, gridDim.x, r, n) ? n : 0;
+            s_rank = r;
+        }
+        __syncthreads();
+        if (s_team == 0) return;
+        rank = s_rank;
+    }
     double sum_res = 0, sum_aux = op.first_aux();
     uint32_t it = 0;
-    // the first tile's units (the same in every iteration); kCluster: the ids of a
+    // kCluster: the first tile's units (the same in every iteration); the ids of a
     // tile's first two units are loaded while the tile before it is summed, those
     // of the first tile before the barrier
     uint32_t first_u = 0, first_ue = 0;
-    if (gw < nfull) {
-        first_u = __ldg(&a.units[gw]);
-        first_ue = __ldg(&a.units[gw + 1]);
+    if (kCluster && rank * kWarps + wid < nfull) {
+        first_u = __ldg(&a.units[rank * kWarps + wid]);
+        first_ue = __ldg(&a.units[rank * kWarps + wid + 1]);
     }
     const uint4 none4 = make_uint4(a.nrows, a.nrows, a.nrows, a.nrows);
     auto ids = [&](uint32_t x, uint32_t end) {
@@ -276,154 +332,12 @@ k_row_solve(SolveArgs a, Op op) {
             __syncthreads();
         }
         double *part = a.partials + (size_t)(it & 1) * 2 * (gridDim.x + nlong);
-        double res = 0, aux = 0;
         auto end_row = [&](uint32_t r, float s, float c, const typename Op::Row &rd, double &rr,
                            double &ra) {
             const float v = op.finish(r, s, c, rd, rr, ra);
             if constexpr (Op::kStore) op.out()[r] = v;
         };
-        uint32_t k = 0;   // class of tile t
-        uint32_t u = first_u, ue = first_ue;
-        for (uint32_t t = gw; t < nfull; t += nw) {
-            while (t >= a.cls.tile0[k + 1]) k++;
-            const uint32_t lg = k == 0 ? 5 : 6 - k;
-            const uint32_t G = 1u << lg;
-            uint32_t r;
-            bool mine;
-            if (k == 0) {
-                r = __ldg(&a.seg_row[t]);
-                mine = false;
-            } else {
-                r = a.cls.row0[k] + (((t - a.cls.tile0[k]) << 5) >> lg) + (lane >> lg);
-                mine = r < a.cls.row0[k + 1] && (lane & (G - 1)) == 0;
-            }
-            typename Op::Row rd{};
-            if (mine) rd = op.row(r);
-            uint32_t nu = 0, nue = 0;   // the next tile's units, one tile ahead
-            if (t + (uint64_t)nw < nfull) {
-                nu = __ldg(&a.units[t + nw]);
-                nue = __ldg(&a.units[t + nw + 1]);
-            }
-            uint4 n0 = none4, n1 = none4;
-            if constexpr (Op::kGather && kCluster) {
-                const bool wrap = t + (uint64_t)nw >= nfull;
-                const uint32_t x = wrap ? first_u : nu, xe = wrap ? first_ue : nue;
-                n0 = ids(x, xe);
-                n1 = ids(x + 1, xe);
-            }
-            Sum2 acc{0, 0};
-            for (; u < ue; u += 2) {   // two units: eight gathers in flight
-                const bool two = u + 1 < ue;   // the same in the whole warp
-                const size_t at = (size_t)u * 32 + lane;
-                float x[8];
-                float4 w0, w1;
-                if constexpr (Op::kGather && kCluster) {
-                    const uint4 j0 = k0, j1 = k1;
-                    k0 = ids(u + 2, ue);
-                    k1 = ids(u + 3, ue);
-                    x[0] = s_val[j0.x];
-                    x[1] = s_val[j0.y];
-                    x[2] = s_val[j0.z];
-                    x[3] = s_val[j0.w];
-                    x[4] = s_val[j1.x];
-                    x[5] = s_val[j1.y];
-                    x[6] = s_val[j1.z];
-                    x[7] = s_val[j1.w];
-                } else if constexpr (Op::kGather) {
-                    const uint4 j0 = __ldcs(&a.idx[at]);
-                    uint4 j1 = none4;
-                    if (two) j1 = __ldcs(&a.idx[at + 32]);
-                    x[0] = row_value(in, j0.x, a.nrows);
-                    x[1] = row_value(in, j0.y, a.nrows);
-                    x[2] = row_value(in, j0.z, a.nrows);
-                    x[3] = row_value(in, j0.w, a.nrows);
-                    if (two) {
-                        x[4] = row_value(in, j1.x, a.nrows);
-                        x[5] = row_value(in, j1.y, a.nrows);
-                        x[6] = row_value(in, j1.z, a.nrows);
-                        x[7] = row_value(in, j1.w, a.nrows);
-                    }
-                }
-                if constexpr (Op::kWeighted) {
-                    w0 = __ldcs(&a.w[at]);
-                    if (two) w1 = __ldcs(&a.w[at + 32]);
-                }
-                auto add4 = [&](const float *v, const float4 &w) {
-                    if constexpr (Op::kGather && Op::kWeighted) {
-                        acc.add(v[0] * w.x, v[1] * w.y);
-                        acc.add(v[2] * w.z, v[3] * w.w);
-                    } else if constexpr (Op::kWeighted) {
-                        acc.add(w.x, w.y);
-                        acc.add(w.z, w.w);
-                    } else {
-                        acc.add(v[0], v[1]);
-                        acc.add(v[2], v[3]);
-                    }
-                };
-                add4(x, w0);
-                if (two) add4(x + 4, w1);
-            }
-            u = nu;
-            ue = nue;
-            if constexpr (Op::kGather && kCluster) {
-                k0 = n0;
-                k1 = n1;
-            }
-            // even and odd steps, then a fixed tree over the row's G lanes
-            float s = low2(acc.s), c = low2(acc.c);
-            pair_add(s, c, high2(acc.s), high2(acc.c));
-            for (uint32_t o = G >> 1; o; o >>= 1) {
-                const float s2 = __shfl_down_sync(kFull, s, o, G);
-                const float c2 = __shfl_down_sync(kFull, c, o, G);
-                pair_add(s, c, s2, c2);
-            }
-            if (k != 0) {
-                if (mine) end_row(r, s, c, rd, res, aux);
-                continue;
-            }
-            // a segment: the last one of its row to finish folds them, lane l
-            // segments l, l + 32, ..., then a fixed tree; the row's partials have
-            // a place of their own (which warp is last is not fixed)
-            const uint32_t first = __ldg(&a.seg_first[r]);
-            const uint32_t nseg = __ldg(&a.seg_first[r + 1]) - first;
-            uint32_t last = 0;
-            if (lane == 0) {
-                // released by the count itself: a full fence would empty this SM's
-                // L1 at every segment; only the last segment's warp acquires
-                __stcg(&a.seg_sum[t], make_float2(s, c));
-                asm volatile("atom.release.gpu.global.inc.u32 %0, [%1], %2;"
-                             : "=r"(last)
-                             : "l"(&a.seg_done[r]), "r"(nseg - 1)
-                             : "memory");
-                last = last == nseg - 1;
-                if (last) __threadfence();
-            }
-            if (!__shfl_sync(kFull, last, 0)) continue;
-            s = 0.0f;
-            c = 0.0f;
-            for (uint32_t q = lane; q < nseg; q += 32) {
-                const float2 v = __ldcg(&a.seg_sum[first + q]);
-                pair_add(s, c, v.x, v.y);
-            }
-#pragma unroll
-            for (int o = 16; o; o >>= 1) {
-                const float s2 = __shfl_down_sync(kFull, s, o);
-                const float c2 = __shfl_down_sync(kFull, c, o);
-                pair_add(s, c, s2, c2);
-            }
-            if (lane == 0) {
-                double rr = 0, ra = 0;
-                end_row(r, s, c, op.row(r), rr, ra);
-                part[2 * (gridDim.x + r)] = rr;
-                part[2 * (gridDim.x + r) + 1] = ra;
-            }
-        }
-        // rows without entries, 32 per tile
-        for (uint32_t t = nfull + gw; t < ntiles; t += nw) {
-            const uint32_t r = a.cls.row0[kRowClasses - 1] + (t - nfull) * 32 + lane;
-            if (r < a.nrows) end_row(r, 0.0f, 0.0f, op.row(r), res, aux);
-        }
-        // this CTA's partials: a tree over each warp, then over the warps
+        // the CTA's sums: a tree over each warp, then over the warps
         auto cta_sum = [&](double &x, double &y) {
 #pragma unroll
             for (int o = 16; o; o >>= 1) {
@@ -445,7 +359,167 @@ k_row_solve(SolveArgs a, Op op) {
                 }
             }
         };
-        cta_sum(res, aux);
+        // this CTA's shares of the grid's work (one, in a full team)
+        double res, aux;
+        for (uint32_t share = rank;;) {
+            const uint32_t gw = share * kWarps + wid;
+            res = 0;
+            aux = 0;
+            uint32_t k = 0;   // class of tile t
+            uint32_t u = first_u, ue = first_ue;
+            if (!kCluster && gw < nfull) {
+                u = __ldg(&a.units[gw]);
+                ue = __ldg(&a.units[gw + 1]);
+            }
+            for (uint32_t t = gw; t < nfull; t += nw) {
+                while (t >= a.cls.tile0[k + 1]) k++;
+                const uint32_t lg = k == 0 ? 5 : 6 - k;
+                const uint32_t G = 1u << lg;
+                uint32_t r;
+                bool mine;
+                if (k == 0) {
+                    r = __ldg(&a.seg_row[t]);
+                    mine = false;
+                } else {
+                    r = a.cls.row0[k] + (((t - a.cls.tile0[k]) << 5) >> lg) + (lane >> lg);
+                    mine = r < a.cls.row0[k + 1] && (lane & (G - 1)) == 0;
+                }
+                typename Op::Row rd{};
+                if (mine) rd = op.row(r);
+                uint32_t nu = 0, nue = 0;   // the next tile's units, one tile ahead
+                if (t + (uint64_t)nw < nfull) {
+                    nu = __ldg(&a.units[t + nw]);
+                    nue = __ldg(&a.units[t + nw + 1]);
+                }
+                uint4 n0 = none4, n1 = none4;
+                if constexpr (Op::kGather && kCluster) {
+                    const bool wrap = t + (uint64_t)nw >= nfull;
+                    const uint32_t x = wrap ? first_u : nu, xe = wrap ? first_ue : nue;
+                    n0 = ids(x, xe);
+                    n1 = ids(x + 1, xe);
+                }
+                Sum2 acc{0, 0};
+                for (; u < ue; u += 2) {   // two units: eight gathers in flight
+                    const bool two = u + 1 < ue;   // the same in the whole warp
+                    const size_t at = (size_t)u * 32 + lane;
+                    float x[8];
+                    float4 w0, w1;
+                    if constexpr (Op::kGather && kCluster) {
+                        const uint4 j0 = k0, j1 = k1;
+                        k0 = ids(u + 2, ue);
+                        k1 = ids(u + 3, ue);
+                        x[0] = s_val[j0.x];
+                        x[1] = s_val[j0.y];
+                        x[2] = s_val[j0.z];
+                        x[3] = s_val[j0.w];
+                        x[4] = s_val[j1.x];
+                        x[5] = s_val[j1.y];
+                        x[6] = s_val[j1.z];
+                        x[7] = s_val[j1.w];
+                    } else if constexpr (Op::kGather) {
+                        const uint4 j0 = __ldcs(&a.idx[at]);
+                        uint4 j1 = none4;
+                        if (two) j1 = __ldcs(&a.idx[at + 32]);
+                        x[0] = row_value(in, j0.x, a.nrows);
+                        x[1] = row_value(in, j0.y, a.nrows);
+                        x[2] = row_value(in, j0.z, a.nrows);
+                        x[3] = row_value(in, j0.w, a.nrows);
+                        if (two) {
+                            x[4] = row_value(in, j1.x, a.nrows);
+                            x[5] = row_value(in, j1.y, a.nrows);
+                            x[6] = row_value(in, j1.z, a.nrows);
+                            x[7] = row_value(in, j1.w, a.nrows);
+                        }
+                    }
+                    if constexpr (Op::kWeighted) {
+                        w0 = __ldcs(&a.w[at]);
+                        if (two) w1 = __ldcs(&a.w[at + 32]);
+                    }
+                    auto add4 = [&](const float *v, const float4 &w) {
+                        if constexpr (Op::kGather && Op::kWeighted) {
+                            acc.add(v[0] * w.x, v[1] * w.y);
+                            acc.add(v[2] * w.z, v[3] * w.w);
+                        } else if constexpr (Op::kWeighted) {
+                            acc.add(w.x, w.y);
+                            acc.add(w.z, w.w);
+                        } else {
+                            acc.add(v[0], v[1]);
+                            acc.add(v[2], v[3]);
+                        }
+                    };
+                    add4(x, w0);
+                    if (two) add4(x + 4, w1);
+                }
+                u = nu;
+                ue = nue;
+                if constexpr (Op::kGather && kCluster) {
+                    k0 = n0;
+                    k1 = n1;
+                }
+                // even and odd steps, then a fixed tree over the row's G lanes
+                float s = low2(acc.s), c = low2(acc.c);
+                pair_add(s, c, high2(acc.s), high2(acc.c));
+                for (uint32_t o = G >> 1; o; o >>= 1) {
+                    const float s2 = __shfl_down_sync(kFull, s, o, G);
+                    const float c2 = __shfl_down_sync(kFull, c, o, G);
+                    pair_add(s, c, s2, c2);
+                }
+                if (k != 0) {
+                    if (mine) end_row(r, s, c, rd, res, aux);
+                    continue;
+                }
+                // a segment: the last one of its row to finish folds them, lane l
+                // segments l, l + 32, ..., then a fixed tree; the row's partials have
+                // a place of their own (which warp is last is not fixed)
+                const uint32_t first = __ldg(&a.seg_first[r]);
+                const uint32_t nseg = __ldg(&a.seg_first[r + 1]) - first;
+                uint32_t last = 0;
+                if (lane == 0) {
+                    // released by the count itself: a full fence would empty this SM's
+                    // L1 at every segment; only the last segment's warp acquires
+                    __stcg(&a.seg_sum[t], make_float2(s, c));
+                    asm volatile("atom.release.gpu.global.inc.u32 %0, [%1], %2;"
+                                 : "=r"(last)
+                                 : "l"(&a.seg_done[r]), "r"(nseg - 1)
+                                 : "memory");
+                    last = last == nseg - 1;
+                    if (last) __threadfence();
+                }
+                if (!__shfl_sync(kFull, last, 0)) continue;
+                s = 0.0f;
+                c = 0.0f;
+                for (uint32_t q = lane; q < nseg; q += 32) {
+                    const float2 v = __ldcg(&a.seg_sum[first + q]);
+                    pair_add(s, c, v.x, v.y);
+                }
+#pragma unroll
+                for (int o = 16; o; o >>= 1) {
+                    const float s2 = __shfl_down_sync(kFull, s, o);
+                    const float c2 = __shfl_down_sync(kFull, c, o);
+                    pair_add(s, c, s2, c2);
+                }
+                if (lane == 0) {
+                    double rr = 0, ra = 0;
+                    end_row(r, s, c, op.row(r), rr, ra);
+                    part[2 * (gridDim.x + r)] = rr;
+                    part[2 * (gridDim.x + r) + 1] = ra;
+                }
+            }
+            // rows without entries, 32 per tile
+            for (uint32_t t = nfull + gw; t < ntiles; t += nw) {
+                const uint32_t r = a.cls.row0[kRowClasses - 1] + (t - nfull) * 32 + lane;
+                if (r < a.nrows) end_row(r, 0.0f, 0.0f, op.row(r), res, aux);
+            }
+            cta_sum(res, aux);
+            if constexpr (kCluster) break;
+            if (threadIdx.x == 0) {
+                part[2 * share] = res;
+                part[2 * share + 1] = aux;
+            }
+            share += s_team;
+            if (share >= gridDim.x) break;
+            __syncthreads();
+        }
         it++;
         if constexpr (kCluster) {
             cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
@@ -486,11 +560,9 @@ k_row_solve(SolveArgs a, Op op) {
         // grid barrier: the last CTA to arrive folds all partials in a fixed order
         // and opens it
         if (threadIdx.x == 0) {
-            part[2 * blockIdx.x] = res;
-            part[2 * blockIdx.x + 1] = aux;
             __threadfence();
             const uint32_t before = atomicAdd(&a.ctl->arrive, 1u);
-            s_state = before + 1 == it * gridDim.x ? 2 : 1;
+            s_state = before + 1 == it * s_team ? 2 : 1;
             __threadfence();
         }
         __syncthreads();
@@ -586,19 +658,19 @@ void choose_form(SolvePlan &p) {
     if (p.cluster) p.cluster = (cluster_runs<Ops>() && ...);
 }
 
-// Launch a solve.  *ctl must be zero but for count.
+// Launch a solve.  *ctl must be zero but for count.  Part of a GPU may have no 16 SMs
+// that can hold a cluster: a small plan takes the other form there.
 template <class Op>
 int launch_solve(const SolvePlan &p, SolveArgs a, Op op, cudaStream_t s) {
-    if (p.cluster) {
+    if (p.cluster && stream_has_whole_gpu(s)) {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr[1];
         cluster_config(&cfg, attr, Op::kGather ? ((size_t)p.n + 4) * 4 : 0, s);
         OLV_CUDA(cudaLaunchKernelEx(&cfg, k_row_solve<Op, true>, a, op));
         return OLV_OK;
     }
-    void *args[] = {&a, &op};
-    OLV_CUDA(cudaLaunchCooperativeKernel((const void *)k_row_solve<Op, false>, dim3(p.grid),
-                                         dim3(kBlock), args, 0, s));
+    k_row_solve<Op, false><<<p.grid, kBlock, 0, s>>>(a, op);
+    OLV_CUDA(cudaGetLastError());
     return OLV_OK;
 }
 

@@ -5,6 +5,7 @@
 
 #include <cub/cub.cuh>
 
+#include "olv_driver.h"
 #include "olv_rowsolve.cuh"
 #include "olv_rowtiles.cuh"
 
@@ -245,6 +246,12 @@ int rows_longer(const uint32_t *sorted_ptr, uint32_t n, const uint32_t *bounds, 
     OLV_CUDA(cudaMemcpyAsync(counts, d.p, (size_t)nb * 4, cudaMemcpyDeviceToHost, s));
     OLV_CUDA(cudaStreamSynchronize(s));
     return OLV_OK;
+}
+
+bool stream_has_whole_gpu(cudaStream_t s) {
+    static const auto green = driver_entry<PFN_cuStreamGetGreenCtx_v12040>("cuStreamGetGreenCtx", 12040);
+    CUgreenCtx c = nullptr;
+    return !green || green(s, &c) != CUDA_SUCCESS || !c;
 }
 
 // First row of every class (RowClassTable::row0) of the sorted rows sptr.
