@@ -14,7 +14,7 @@
 // All iterations run in one launch.  Small structures (at most kClusterRows
 // rows and kClusterEntries entries) take one thread-block cluster of 16 CTAs:
 // every CTA copies all gathered values to shared memory at the start of an
-// iteration (16 SMs read at most 217 KB each, contiguous), where 32 gathers take
+// iteration (at most 32 KB, contiguous), where 32 gathers take
 // 3-4 cycles of bank conflicts instead of 32 lookups in L1, and the barrier
 // between two iterations is the cluster's.  Larger ones take the whole GPU (join_team
 // below): at the grid barrier the last CTA to arrive adds up the
@@ -23,10 +23,9 @@
 // to L2 and an SM sends one per cycle, so as many warps as possible keep eight
 // gathers per lane in flight, the index loads cost 4 requests per 128 entries,
 // and no fence (which would empty L1) stands inside an iteration.
-// Measured: PageRank on a uniform digraph of 20,011 vertices, 50 iterations, 640
-// -> 440 us (a cluster; an iteration is 1 us of copying, 4 us of sums bound by
-// instructions, 2 us of barrier and fold); weighted PageRank on RMAT-20, 100
-// sweeps and their adjoint, 20.2 -> 12.7 ms.  A copy of only the most gathered
+// Measured: PageRank on a uniform digraph of 20,011 vertices, 50 iterations, 600
+// -> 374 us; weighted PageRank on RMAT-20, 100 sweeps and their adjoint, 20.2 ->
+// 12.7 ms.  A copy of only the most gathered
 // values (16 to 217 KB of shared memory) in the whole-GPU form was slower at
 // every size: a gather in flight holds a line of L1, which the copy takes away.
 //
@@ -102,8 +101,16 @@ struct Sum2 {
 };
 
 constexpr int kClusterCTAs = 16, kClusterThreads = 1024;
-constexpr uint32_t kClusterRows = 53 * 1024;       // 217 KB of shared memory
-constexpr uint32_t kClusterEntries = 2u << 20;
+// Structures of at most so many rows and entries take one cluster.  Above, the copy of
+// the values and 16 SMs' share of the entries cost more than the grid barrier.
+// PageRank / weighted PageRank (forward and adjoint), 20 iterations, us, one cluster
+// against the whole GPU: RMAT of 4096 vertices, 53 K edges 157 / 450 against 192 / 490,
+// 171 K edges 191 / 528 against 233 / 597; uniform digraphs of 8000 vertices, 32 K edges
+// 147 / 384 against 159 / 416, 200 K 174 / 484 against 184 / 461, 391 K 203 / 556 against
+// 209 / 524, 1 M 424 / 1090 against 268 / 680; of 30,000 vertices, 210 K edges 210 / 543
+// against 179 / 473; of 54,000, 108 K edges 261 / 684 against 175 / 462.
+constexpr uint32_t kClusterRows = 8192;       // 32 KB of shared memory
+constexpr uint32_t kClusterEntries = 3u << 16;
 constexpr uint32_t kRowLong = 2048;    // rows with more entries are segmented
 constexpr uint32_t kRowSeg = 512;      // entries per segment
 constexpr int kRowClasses = 8;         // segments, 32..1 lanes per row, empty rows
@@ -273,6 +280,7 @@ k_row_solve(SolveArgs a, Op op) {
     __shared__ double s_part[2][2];   // kCluster: this CTA's sums, by iteration parity
     __shared__ uint32_t s_state;   // barrier: 0 out of time, 1 open, 2 this CTA is the last
     __shared__ uint32_t s_rank, s_team;   // !kCluster: this CTA in its team, CTAs in it
+    __shared__ uint2 s_first[kWarps];     // !kCluster: units of the warps' first tiles
     constexpr unsigned kFull = 0xffffffffu;
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t nw = gridDim.x * kWarps;
@@ -281,9 +289,11 @@ k_row_solve(SolveArgs a, Op op) {
     uint32_t rank = blockIdx.x;
     if constexpr (!kCluster) {
         if (threadIdx.x == 0) {
-            uint32_t r, n;
+            uint32_t r, n = 0;
             s_team = join_team(a.ctl, gridDim.x, r, n) ? n : 0;
-            s_rank = r;
+            // a full team by CTA number: neighbours are on different SMs, so each SM gets
+            // its share of the CTAs with a tile more (by order of arrival: 5-9 % slower)
+            s_rank = n == gridDim.x ? blockIdx.x : r;
         }
         __syncthreads();
         if (s_team == 0) return;
@@ -291,14 +301,16 @@ k_row_solve(SolveArgs a, Op op) {
     }
     double sum_res = 0, sum_aux = op.first_aux();
     uint32_t it = 0;
-    // kCluster: the first tile's units (the same in every iteration); the ids of a
+    // the first tile's units (the same in every iteration); kCluster: the ids of a
     // tile's first two units are loaded while the tile before it is summed, those
     // of the first tile before the barrier
     uint32_t first_u = 0, first_ue = 0;
-    if (kCluster && rank * kWarps + wid < nfull) {
+    if (rank * kWarps + wid < nfull) {
         first_u = __ldg(&a.units[rank * kWarps + wid]);
         first_ue = __ldg(&a.units[rank * kWarps + wid + 1]);
     }
+    if constexpr (!kCluster) s_first[wid] = make_uint2(first_u, first_ue);   // not in registers
+    __syncwarp();
     const uint4 none4 = make_uint4(a.nrows, a.nrows, a.nrows, a.nrows);
     auto ids = [&](uint32_t x, uint32_t end) {
         return x < end ? __ldg(&a.idx[(size_t)x * 32 + lane]) : none4;
@@ -367,9 +379,13 @@ k_row_solve(SolveArgs a, Op op) {
             aux = 0;
             uint32_t k = 0;   // class of tile t
             uint32_t u = first_u, ue = first_ue;
-            if (!kCluster && gw < nfull) {
-                u = __ldg(&a.units[gw]);
-                ue = __ldg(&a.units[gw + 1]);
+            if constexpr (!kCluster) {
+                u = s_first[wid].x;
+                ue = s_first[wid].y;
+                if (share >= s_team && gw < nfull) {   // not this CTA's first share
+                    u = __ldg(&a.units[gw]);
+                    ue = __ldg(&a.units[gw + 1]);
+                }
             }
             for (uint32_t t = gw; t < nfull; t += nw) {
                 while (t >= a.cls.tile0[k + 1]) k++;
@@ -632,20 +648,20 @@ inline void cluster_config(cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr, s
     cfg->numAttrs = 1;
 }
 
-// Whether the GPU runs the cluster form of Op at its largest.  The attributes belong
-// to the kernel, whatever handle or thread launches it, so they are set to the most
-// that any plan needs and never lowered.
+// Whether the GPU runs the cluster form of Op at its largest.  (Its shared memory stays
+// below the 48 KB that need no attribute: one set to each handle's size belongs to the
+// kernel, and threads undid each other's.)
 template <class Op>
 bool cluster_runs() {
     const void *fn = (const void *)k_row_solve<Op, true>;
-    const int smem = Op::kGather ? (int)((kClusterRows + 4) * 4) : 0;
+    constexpr size_t smem = Op::kGather ? (kClusterRows + 4) * 4 : 0;
+    static_assert(smem <= 47 * 1024, "one set of launch attributes for all plans");
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
-    cluster_config(&cfg, attr, (size_t)smem, nullptr);
+    cluster_config(&cfg, attr, smem, nullptr);
     int n = 0;
     const bool ok =
         cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
         cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess && n >= 1;
     if (!ok) cudaGetLastError();
     return ok;

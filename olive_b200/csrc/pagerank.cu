@@ -22,14 +22,11 @@
 //     folded in a fixed order and decide convergence on the device.
 //
 // Two ways to run the iterations.  All of them in one launch (olv_rowsolve.cuh)
-// where launches and the loop around them were most of the time (below
-// kPrSolveEdges edges), and on graphs without a segmented row of any size; else
-// an iteration is a tile pass and a one-CTA fold inside a CUDA graph
-// (olv_rowtiles.cuh), which reads the hubs' rows faster (no counts and fences
-// among the gathers).  Both measured, us for 20 iterations, tile pass / one
-// launch: RMAT-12 316 / 168, RMAT-16 457 / 363, RMAT-18 (3.9 M edges) 516 / 536,
-// RMAT-19 735 / 942, RMAT-21 2265 / 3070; uniform digraphs of 16 edges a vertex,
-// 2^16 vertices 343 / 264, 2^18 624 / 520, 2^21 3181 / 2912.
+// where launches and the loop around them were most of the time, and on graphs
+// without a segmented row that have work enough per row; else an iteration is a tile
+// pass and a one-CTA fold inside a CUDA graph (olv_rowtiles.cuh), which reads the hubs'
+// rows faster (no counts and fences among the gathers) and passes over rows of few
+// entries faster.  The line is one_launch()'s.
 #include <algorithm>
 #include <vector>
 
@@ -42,7 +39,6 @@
 namespace olv {
 
 constexpr int kRedThreads = 1024;   // 32 warps: one more tree over them
-constexpr uint64_t kPrSolveEdges = 3u << 20;
 
 struct PrCtl {
     double base;        // (1-alpha)/N + alpha*d/N for the running iteration
@@ -258,9 +254,28 @@ struct PrPlan {
     }
 };
 
+// One launch for all iterations, or a pass each.  Measured from one build, us for 20
+// iterations, one launch / a pass each:
+//   uniform digraphs, edges a vertex: 2^17 vertices, 2: 211 / 268, 8: 273 / 307;
+//   262,144, 1: 310 / 285, 3: 345 / 304, 4: 328 / 329, 8: 358 / 408; 524,288, 1: 399 /
+//   332, 4: 413 / 430, 12: 726 / 773; 1,000,003, 1: 579 / 418, 2: 559 / 496, 4: 613 /
+//   603, 8: 861 / 875; 2,000,003, 1: 903 / 620, 2: 891 / 739; 2^21, 16: 2932 / 3181;
+//   grids of 490,000 and 4 M vertices 265 / 342, 929 / 1265;
+//   RMAT, edges drawn a vertex: 2^16, 16: 346 / 420; 2^17, 4: 308 / 451, 16: 497 / 519,
+//   24 (2.9 M edges): 516 / 456; 200,003, 8: 475 / 446; 2^18, 1: 314 / 426, 8: 534 / 513,
+//   12 (3 M): 611 / 563; 300,007, 1: 436 / 330, 8 (1.3 M): 393 / 501, 16: 580 / 481;
+//   370,001, 4 (1 M): 541 / 452, 8 (2 M): 430 / 527, 16: 621 / 538; 440,009, 8 (2.9 M):
+//   732 / 595; 2^19, 2: 647 / 560, 8: 817 / 638; 2^20, 16: 1611 / 1117.
+static bool one_launch(const olv_graph *g) {
+    const bool few = g->E < 2u << 20;
+    if (few && g->V <= 1u << 18) return true;
+    const bool rows_long_enough = 2 * g->E >= 7 * (uint64_t)g->V;
+    return rows_long_enough && (g->max_in_degree <= kRowLong || (few && g->V <= 3u << 17));
+}
+
 static int build_pr_plan(olv_graph *g, PrPlan &p) {
     const uint32_t V = g->V;
-    p.solve = g->E < kPrSolveEdges || g->max_in_degree <= kRowLong;
+    p.solve = one_launch(g);
     if (p.solve) {
         OLV_TRY(build_solve_plan(g->colptr.as<uint32_t>(), g->rowidx.as<uint32_t>(), nullptr, V,
                                  g->E, g->tune.pr_tile_u, false, g->num_sms, g->stream, p.sp));
