@@ -20,6 +20,7 @@
 //     L1 change (FP64) is below tol.
 #include <algorithm>
 #include <numeric>
+#include <type_traits>
 #include <vector>
 
 #include <cooperative_groups.h>
@@ -54,7 +55,7 @@ struct BatchArgs {
     int32_t *levels;             // [V]
     float *ppr, *ppr_tmp;        // [V][K]
     float *inv_deg;              // [V] 1 / out-degree (0: dangling), written per PPR item
-    uint2 *ew;                   // [E] in-edges as (local source, its inverse degree), K % 4 == 0
+    uint2 *ew;                   // rows of four vectors: [E] in-edges as (local source, its inverse degree)
     uint32_t n_large;            // items order[0 .. n_large) are a cluster's, the rest a CTA's
     uint32_t *counter;           // work queue head
     uint32_t *ppr_iters;         // [count]
@@ -428,25 +429,10 @@ __device__ void team_ppr(const BatchArgs &a, uint32_t inst, uint32_t C, uint32_t
     sync();   // shared state and vectors are the next item's
 }
 
-// Whether an item's sweeps can use rows of four vectors per lane.
-__device__ __forceinline__ bool ppr_rows(const BatchArgs &a) {
-    return a.ew != nullptr;
-}
-
-template <class Sync, class At>
-__device__ __forceinline__ void team_ppr_k(const BatchArgs &a, uint32_t inst, uint32_t C,
-                                           uint32_t rank, Sync sync, At at, RowsShared &sh) {
-    switch (a.K) {
-        case 32: team_ppr<8>(a, inst, C, rank, sync, at, sh); break;
-        case 16: team_ppr<4>(a, inst, C, rank, sync, at, sh); break;
-        case 8: team_ppr<2>(a, inst, C, rank, sync, at, sh); break;
-        default: team_ppr<1>(a, inst, C, rank, sync, at, sh); break;
-    }
-}
-
 // The same by this CTA alone.
+template <int L>
 __device__ __forceinline__ void cta_rows_ppr(const BatchArgs &a, uint32_t inst, RowsShared &sh) {
-    team_ppr_k(
+    team_ppr<L>(
         a, inst, 1, 0, [] { __syncthreads(); }, [](auto *p, uint32_t) { return p; }, sh);
 }
 
@@ -503,9 +489,12 @@ __device__ void cta_ppr(const BatchArgs &a, uint32_t inst) {
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(kBatchThreads) k_batch(BatchArgs a) {
+// L (here and below): lanes per vertex of the rows of four vectors per lane, 0: a lane
+// per vector.  Kernels of their own: with all sweeps in one, the registers of the
+// others made the lane-per-vector sweep spill (K = 1 and 12: up to 1.4x slower).
+template <int L>
+__global__ void __launch_bounds__(kBatchThreads, 2) k_batch(BatchArgs a) {
     __shared__ uint32_t bm[3 * (kBatchMaxV / 32)];
-    __shared__ RowsShared rows;
     __shared__ uint32_t s_item;
     const uint32_t n_items = (uint32_t)a.count * a.tasks;
     for (;;) {
@@ -516,12 +505,14 @@ __global__ void __launch_bounds__(kBatchThreads) k_batch(BatchArgs a) {
         if (item >= n_items) break;
         const uint32_t inst = a.order[item / a.tasks];
         const bool bfs = a.tasks == 2 ? (item % 2 == 0) : (a.do_bfs != 0);
-        if (bfs)
+        if (bfs) {
             cta_bfs(a, inst, bm);
-        else if (ppr_rows(a))
-            cta_rows_ppr(a, inst, rows);
-        else
+        } else if constexpr (L != 0) {
+            __shared__ RowsShared rows;
+            cta_rows_ppr<L>(a, inst, rows);
+        } else {
             cta_ppr(a, inst);
+        }
     }
 }
 
@@ -609,12 +600,10 @@ __device__ void cluster_ppr(const BatchArgs &a, uint32_t inst, cg::cluster_group
     if (lane == 0 && visits) atomicAdd(&a.stats[1], visits * (unsigned long long)K);
 }
 
+template <int L>
 __global__ void __launch_bounds__(kClusterThreads, 1) k_batch_cluster(BatchArgs a) {
     __shared__ uint32_t bm[3 * (kBatchMaxV / 32)];
-    __shared__ union {
-        ClusterShared one;   // a lane per vector
-        RowsShared rows;     // four vectors per lane
-    } sh;
+    __shared__ std::conditional_t<L != 0, RowsShared, ClusterShared> sh;
     __shared__ uint32_t s_item;
     cg::cluster_group cl = cg::this_cluster();
     // the cluster's items first, largest first (counter[1], taken by CTA 0), then
@@ -625,23 +614,25 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_batch_cluster(BatchArgs 
             cl.sync();
             const uint32_t item = *cl.map_shared_rank(&s_item, 0);
             if (item >= a.n_large) break;
-            if (ppr_rows(a))
-                team_ppr_k(
+            if constexpr (L != 0)
+                team_ppr<L>(
                     a, a.order[item], cl.num_blocks(), cl.block_rank(), [&] { cl.sync(); },
-                    [&](auto *p, uint32_t r) { return cl.map_shared_rank(p, r); }, sh.rows);
+                    [&](auto *p, uint32_t r) { return cl.map_shared_rank(p, r); }, sh);
             else
-                cluster_ppr(a, a.order[item], cl, sh.one);
+                cluster_ppr(a, a.order[item], cl, sh);
         }
         cl.sync();   // the last item's number has been read by every CTA
-        for (;;) {
+        if constexpr (L != 0) {
+            for (;;) {
+                __syncthreads();
+                if (threadIdx.x == 0) s_item = a.n_large + atomicAdd(&a.counter[2], 1u);
+                __syncthreads();
+                const uint32_t item = s_item;
+                if (item >= (uint32_t)a.count) break;
+                cta_rows_ppr<L>(a, a.order[item], sh);
+            }
             __syncthreads();
-            if (threadIdx.x == 0) s_item = a.n_large + atomicAdd(&a.counter[2], 1u);
-            __syncthreads();
-            const uint32_t item = s_item;
-            if (item >= (uint32_t)a.count) break;
-            cta_rows_ppr(a, a.order[item], sh.rows);
         }
-        __syncthreads();
     }
     if (a.do_bfs) {   // BFS items: one CTA each (counter[0])
         for (;;) {
@@ -656,13 +647,22 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_batch_cluster(BatchArgs 
     cl.sync();   // no CTA leaves while another may still read its shared memory
 }
 
+using BatchKernel = void (*)(BatchArgs);
+static BatchKernel batch_kernel(const BatchArgs &a, BatchKernel k32, BatchKernel k16, BatchKernel k8,
+                                BatchKernel k4, BatchKernel other) {
+    if (!a.ew) return other;
+    return a.K == 32 ? k32 : a.K == 16 ? k16 : a.K == 8 ? k8 : k4;
+}
+
 // Launch k_batch_cluster with `want` CTAs per cluster (8 or 16), or with the
 // largest size the GPU runs when want = 1; one CTA per SM.  *launched =
 // false when no wanted size is available.
 static int launch_batch_cluster(const BatchArgs &a, int num_sms, cudaStream_t s, int want,
                                 bool *launched, int *cluster_size) {
     *launched = false;
-    if (cudaFuncSetAttribute(k_batch_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+    const auto kernel = batch_kernel(a, k_batch_cluster<8>, k_batch_cluster<4>, k_batch_cluster<2>,
+                                     k_batch_cluster<1>, k_batch_cluster<0>);
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
         cudaSuccess)
         cudaGetLastError();
     for (int C : {16, 8}) {
@@ -680,12 +680,12 @@ static int launch_batch_cluster(const BatchArgs &a, int num_sms, cudaStream_t s,
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int ncl = 0;
-        if (cudaOccupancyMaxActiveClusters(&ncl, k_batch_cluster, &cfg) != cudaSuccess || ncl < 1) {
+        if (cudaOccupancyMaxActiveClusters(&ncl, kernel, &cfg) != cudaSuccess || ncl < 1) {
             cudaGetLastError();
             continue;
         }
         cfg.gridDim = dim3(C * std::min(ncl, std::max(1, num_sms / C)));
-        OLV_CUDA(cudaLaunchKernelEx(&cfg, k_batch_cluster, a));
+        OLV_CUDA(cudaLaunchKernelEx(&cfg, kernel, a));
         *launched = true;
         *cluster_size = C;
         return OLV_OK;
@@ -825,10 +825,11 @@ extern "C" int olv_batch_run(olv_graph *g, const uint32_t *inst_offsets, int cou
     if (g->tune.batch_cluster)
         OLV_TRY(launch_batch_cluster(a, g->num_sms, s, g->tune.batch_cluster, &launched, &csize));
     if (!launched) {   // one CTA per item
+        const auto kernel = batch_kernel(a, k_batch<8>, k_batch<4>, k_batch<2>, k_batch<1>, k_batch<0>);
         int per_sm = 0;
-        OLV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch, kBatchThreads, 0));
+        OLV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBatchThreads, 0));
         const int grid = std::max(1, per_sm) * g->num_sms;
-        k_batch<<<grid, kBatchThreads, 0, s>>>(a);
+        kernel<<<grid, kBatchThreads, 0, s>>>(a);
     }
     OLV_CUDA(cudaGetLastError());
     OLV_CUDA(cudaEventRecord(g->ev1, s));
