@@ -36,11 +36,9 @@ constexpr int kBatchThreads = 512;
 constexpr uint32_t kBatchMaxV = 65536;
 constexpr int kBatchWarps = kBatchThreads / 32;
 constexpr int kBatchMaxWarps = 32;
-// PPR items of at most this many vertices take one CTA, larger ones a cluster: a
-// sweep of a small instance on 16 CTAs is mostly its barrier, while a larger one on a
-// CTA is left running alone at the end.  The line at 512 / 1024 / 2048 / 4096, K = 32,
-// 20 sweeps: 512 instances of 50..2000 vertices 5.5 / 4.1 / 2.0 / - ms, 64 of 300..9001
-// 1.88 / 1.94 / 2.31 / 2.65, 96 of 1024..65536 11.6 / 11.6 / 11.6 / 12.5.
+// PPR items of at most this many vertices can take one CTA, larger ones take a
+// cluster (choose_large() below): a sweep of a small instance on 16 CTAs is mostly its
+// barrier, while a larger one on a CTA is left running alone at the end.
 constexpr uint32_t kCtaItem = 2048;
 
 struct BatchArgs {
@@ -236,7 +234,7 @@ constexpr double kDangOne = 4611686018427387904.0;   // 2^62
 
 struct alignas(16) RowsShared {
     unsigned long long dang[3][32];       // this CTA's dangling mass, by sweep modulo 3
-    double warp_res[kBatchMaxWarps][32];  // per warp and vector
+    double warp_res[2][kBatchMaxWarps][32];   // per warp and vector, by sweep parity
     double res[2][32];                    // this CTA's L1 change, by sweep parity
     alignas(16) uint32_t seed[32];
     alignas(16) float tele[32];           // what a seed gets in this sweep
@@ -244,7 +242,8 @@ struct alignas(16) RowsShared {
 };
 
 // One sweep of one warp over the vertex groups g = w0, w0 + nw, ...; adds the new
-// dangling mass to dang (shared) and, kRes, the L1 change to res.
+// dangling mass to dang (shared) and, kRes, the L1 change to res: a group's by a fixed
+// tree over its vertices, then the groups in order.
 template <int L, bool kRes>
 __device__ __forceinline__ void ppr_sweep_rows(const BatchArgs &a, const PprView &p,
                                                const RowsShared &sh, uint32_t lane, uint32_t w0,
@@ -291,6 +290,7 @@ __device__ __forceinline__ void ppr_sweep_rows(const BatchArgs &a, const PprView
                 acc.w = fmaf(x[r].w, w[r], acc.w);
             }
         }
+        double change[4] = {0.0, 0.0, 0.0, 0.0};
         if (valid) {
             const uint4 sd = reinterpret_cast<const uint4 *>(sh.seed)[q];
             float4 t = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -302,10 +302,10 @@ __device__ __forceinline__ void ppr_sweep_rows(const BatchArgs &a, const PprView
             const float4 nv = make_float4(fmaf(p.alpha, acc.x, t.x), fmaf(p.alpha, acc.y, t.y),
                                           fmaf(p.alpha, acc.z, t.z), fmaf(p.alpha, acc.w, t.w));
             if (kRes) {
-                res[0] += fabs((double)nv.x - (double)old.x);
-                res[1] += fabs((double)nv.y - (double)old.y);
-                res[2] += fabs((double)nv.z - (double)old.z);
-                res[3] += fabs((double)nv.w - (double)old.w);
+                change[0] = fabs((double)nv.x - (double)old.x);
+                change[1] = fabs((double)nv.y - (double)old.y);
+                change[2] = fabs((double)nv.z - (double)old.z);
+                change[3] = fabs((double)nv.w - (double)old.w);
             }
             dst4[(size_t)v * L] = nv;
             if (inv == 0.0f) {   // a dangling vertex: rare enough for shared atomics
@@ -314,6 +314,15 @@ __device__ __forceinline__ void ppr_sweep_rows(const BatchArgs &a, const PprView
                 atomicAdd(&dang[4 * q + 2], __double2ull_rn((double)nv.z * kDangOne));
                 atomicAdd(&dang[4 * q + 3], __double2ull_rn((double)nv.w * kDangOne));
             }
+        }
+        if (kRes) {
+#pragma unroll
+            for (int o = L; o < 32; o <<= 1)
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+                    change[c] += __shfl_xor_sync(0xffffffffu, change[c], o);
+#pragma unroll
+            for (int c = 0; c < 4; c++) res[c] += change[c];
         }
     }
 }
@@ -328,6 +337,10 @@ __device__ void team_ppr(const BatchArgs &a, uint32_t inst, uint32_t C, uint32_t
     const uint32_t gw = rank * warps + wid, nw = C * warps, q = lane % L;
     const PprView p = ppr_view(a, inst, lane);
     const bool with_res = a.tol > 0.0;   // nothing is below a tolerance of zero
+    // a cluster's warps have a group each of an item that can be a CTA's: the L1 change is
+    // added up as that CTA's warps would (each its groups in order), so that the sweep
+    // at which an item stops does not depend on the team
+    const bool as_cta = C > 1 && p.n <= kCtaItem;
     // start vectors and inverse degrees, then the in-edges as pairs
     const uint32_t tid = rank * blockDim.x + threadIdx.x, nt = C * blockDim.x;
     for (uint32_t v = tid; v < p.n; v += nt) {
@@ -385,29 +398,35 @@ __device__ void team_ppr(const BatchArgs &a, uint32_t inst, uint32_t C, uint32_t
         else
             ppr_sweep_rows<L, false>(a, p, sh, lane, gw, nw, src, dst, dang, res);
         if (with_res) {
-            // the warp's slots by a fixed tree, then the CTA's warps in order
-#pragma unroll
-            for (int o = L; o < 32; o <<= 1)
-#pragma unroll
-                for (int c = 0; c < 4; c++) res[c] += __shfl_xor_sync(kFull, res[c], o);
             if (lane < L)
 #pragma unroll
-                for (int c = 0; c < 4; c++) sh.warp_res[wid][4 * q + c] = res[c];
-            __syncthreads();
-            if (wid == 0) {
-                double t = 0.0;
-                if ((int)lane < p.K)
-                    for (uint32_t w = 0; w < warps; w++) t += sh.warp_res[w][lane];
-                sh.res[pb][lane] = t;
+                for (int c = 0; c < 4; c++) sh.warp_res[pb][wid][4 * q + c] = res[c];
+            if (!as_cta) {   // this CTA's warps in order
+                __syncthreads();
+                if (wid == 0) {
+                    double t = 0.0;
+                    if ((int)lane < p.K)
+                        for (uint32_t w = 0; w < warps; w++) t += sh.warp_res[pb][w][lane];
+                    sh.res[pb][lane] = t;
+                }
             }
         }
         // orders this sweep's writes (vectors and sums) before the next sweep's reads
         sync();
         it++;
         if (with_res) {   // stop test: the same on every CTA
+            if (as_cta) {   // (no CTA reads the last sweep's sums any more)
+                double t = 0.0;
+                for (uint32_t r = 0; r < C; r++) t += at(&sh.warp_res[pb][wid][0], r)[lane];
+                sh.warp_res[pb ^ 1][wid][lane] = t;
+                __syncthreads();
+            }
             if (wid == 0) {
                 double t = 0.0;
-                for (uint32_t r = 0; r < C; r++) t += at(&sh.res[pb][0], r)[lane];
+                if (as_cta)
+                    for (uint32_t w = 0; w < warps; w++) t += sh.warp_res[pb ^ 1][w][lane];
+                else
+                    for (uint32_t r = 0; r < C; r++) t += at(&sh.res[pb][0], r)[lane];
                 double mx = (int)lane < p.K ? t : 0.0;
 #pragma unroll
                 for (int o = 16; o; o >>= 1) mx = fmax(mx, __shfl_xor_sync(kFull, mx, o));
@@ -494,7 +513,10 @@ __device__ void cta_ppr(const BatchArgs &a, uint32_t inst) {
 // others made the lane-per-vector sweep spill (K = 1 and 12: up to 1.4x slower).
 template <int L>
 __global__ void __launch_bounds__(kBatchThreads, 2) k_batch(BatchArgs a) {
-    __shared__ uint32_t bm[3 * (kBatchMaxV / 32)];
+    __shared__ union {
+        uint32_t bm[3 * (kBatchMaxV / 32)];
+        std::conditional_t<L != 0, RowsShared, char> rows;
+    } mem;
     __shared__ uint32_t s_item;
     const uint32_t n_items = (uint32_t)a.count * a.tasks;
     for (;;) {
@@ -506,10 +528,9 @@ __global__ void __launch_bounds__(kBatchThreads, 2) k_batch(BatchArgs a) {
         const uint32_t inst = a.order[item / a.tasks];
         const bool bfs = a.tasks == 2 ? (item % 2 == 0) : (a.do_bfs != 0);
         if (bfs) {
-            cta_bfs(a, inst, bm);
+            cta_bfs(a, inst, mem.bm);
         } else if constexpr (L != 0) {
-            __shared__ RowsShared rows;
-            cta_rows_ppr<L>(a, inst, rows);
+            cta_rows_ppr<L>(a, inst, mem.rows);
         } else {
             cta_ppr(a, inst);
         }
@@ -602,8 +623,11 @@ __device__ void cluster_ppr(const BatchArgs &a, uint32_t inst, cg::cluster_group
 
 template <int L>
 __global__ void __launch_bounds__(kClusterThreads, 1) k_batch_cluster(BatchArgs a) {
-    __shared__ uint32_t bm[3 * (kBatchMaxV / 32)];
-    __shared__ std::conditional_t<L != 0, RowsShared, ClusterShared> sh;
+    __shared__ union {
+        std::conditional_t<L != 0, RowsShared, ClusterShared> sh;
+        uint32_t bm[3 * (kBatchMaxV / 32)];   // BFS, after the PPR items
+    } mem;
+    auto &sh = mem.sh;
     __shared__ uint32_t s_item;
     cg::cluster_group cl = cg::this_cluster();
     // the cluster's items first, largest first (counter[1], taken by CTA 0), then
@@ -641,7 +665,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) k_batch_cluster(BatchArgs 
             const uint32_t item = s_item;
             __syncthreads();
             if (item >= (uint32_t)a.count) break;
-            cta_bfs(a, a.order[item], bm);
+            cta_bfs(a, a.order[item], mem.bm);
         }
     }
     cl.sync();   // no CTA leaves while another may still read its shared memory
@@ -654,11 +678,49 @@ static BatchKernel batch_kernel(const BatchArgs &a, BatchKernel k32, BatchKernel
     return a.K == 32 ? k32 : a.K == 16 ? k16 : a.K == 8 ? k8 : k4;
 }
 
+// Which of the items (sizes, largest first) the clusters take: those above kCtaItem,
+// and of the others the largest ones where that ends the call earlier.  The times are
+// estimates in ns a sweep.  An item takes a cluster a barrier, a chain of loads of its
+// row's length, and a thirtieth of its work; a CTA its work, per vertex and per in-edge
+// (measured: K = 4..32, 60..4000 vertices, 2..24 in-edges each, within about 30 %).  The
+// clusters' items come first, then the CTAs take the rest, which ends with the largest
+// or when all CTAs have had their share.  20 sweeps, K = 32, equal items of eight
+// in-edges a vertex, all on clusters / all on CTAs, us: one of 250 vertices 152 / 151, of
+// 2000 166 / 769; 28 of 250 424 / 167, of 2000 514 / 788; 96 of 2000 1471 / 801.
+static uint32_t choose_large(const std::vector<uint32_t> &sizes, double deg, int K, int C,
+                             int clusters) {
+    const size_t count = sizes.size();
+    size_t m = 0;
+    while (m < count && sizes[m] > kCtaItem) m++;
+    // the smaller ones' sums need a group of vertices a warp (team_ppr)
+    if ((uint64_t)C * (kClusterThreads / 32) * (128 / K) < kCtaItem) return (uint32_t)m;
+    auto cta = [&](size_t i) { return sizes[i] * (0.22 * K + (0.4 + 0.025 * K) * deg); };
+    auto cluster = [&](size_t i) { return 3000.0 + deg * (130.0 + 1200.0 / K) + cta(i) / 30; };
+    std::vector<double> busy(clusters, 0.0);   // until when each cluster is
+    auto give = [&](size_t i) { *std::min_element(busy.begin(), busy.end()) += cluster(i); };
+    double rest = 0, best = 0;
+    for (size_t i = 0; i < m; i++) give(i);
+    for (size_t i = m; i < count; i++) rest += cta(i);
+    uint32_t at = (uint32_t)m;
+    for (size_t i = m;; i++) {   // items [0, i) on clusters
+        const double end = *std::max_element(busy.begin(), busy.end()) +
+                           (i < count ? std::max(cta(i), rest / (clusters * C)) : 0.0);
+        if (i == m || end < best) {
+            best = end;
+            at = (uint32_t)i;
+        }
+        if (i == count) return at;
+        give(i);
+        rest -= cta(i);
+    }
+}
+
 // Launch k_batch_cluster with `want` CTAs per cluster (8 or 16), or with the
 // largest size the GPU runs when want = 1; one CTA per SM.  *launched =
 // false when no wanted size is available.
-static int launch_batch_cluster(const BatchArgs &a, int num_sms, cudaStream_t s, int want,
-                                bool *launched, int *cluster_size) {
+static int launch_batch_cluster(BatchArgs a, const std::vector<uint32_t> &sizes, double deg,
+                                int num_sms, cudaStream_t s, int want, bool *launched,
+                                int *cluster_size) {
     *launched = false;
     const auto kernel = batch_kernel(a, k_batch_cluster<8>, k_batch_cluster<4>, k_batch_cluster<2>,
                                      k_batch_cluster<1>, k_batch_cluster<0>);
@@ -684,7 +746,9 @@ static int launch_batch_cluster(const BatchArgs &a, int num_sms, cudaStream_t s,
             cudaGetLastError();
             continue;
         }
-        cfg.gridDim = dim3(C * std::min(ncl, std::max(1, num_sms / C)));
+        ncl = std::min(ncl, std::max(1, num_sms / C));
+        cfg.gridDim = dim3(C * ncl);
+        a.n_large = a.ew ? choose_large(sizes, deg, a.K, C, ncl) : (uint32_t)a.count;
         OLV_CUDA(cudaLaunchKernelEx(&cfg, kernel, a));
         *launched = true;
         *cluster_size = C;
@@ -807,13 +871,8 @@ extern "C" int olv_batch_run(olv_graph *g, const uint32_t *inst_offsets, int cou
         rows = false;
     }
     a.ew = rows ? bs.ew.as<uint2>() : nullptr;
-    a.n_large = (uint32_t)count;
-    if (rows) {
-        a.n_large = 0;
-        while (a.n_large < (uint32_t)count &&
-               off[order[a.n_large] + 1] - off[order[a.n_large]] > kCtaItem)
-            a.n_large++;
-    }
+    std::vector<uint32_t> sizes(count);
+    for (int i = 0; i < count; i++) sizes[i] = off[order[i] + 1] - off[order[i]];
     a.counter = bs.counter.as<uint32_t>();
     a.ppr_iters = bs.iters.as<uint32_t>();
     a.stats = bs.stats.as<unsigned long long>();
@@ -823,7 +882,8 @@ extern "C" int olv_batch_run(olv_graph *g, const uint32_t *inst_offsets, int cou
     bool launched = false;
     int csize = 0;
     if (g->tune.batch_cluster)
-        OLV_TRY(launch_batch_cluster(a, g->num_sms, s, g->tune.batch_cluster, &launched, &csize));
+        OLV_TRY(launch_batch_cluster(a, sizes, (double)g->E / g->V, g->num_sms, s,
+                                     g->tune.batch_cluster, &launched, &csize));
     if (!launched) {   // one CTA per item
         const auto kernel = batch_kernel(a, k_batch<8>, k_batch<4>, k_batch<2>, k_batch<1>, k_batch<0>);
         int per_sm = 0;
