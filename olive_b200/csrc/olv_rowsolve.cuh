@@ -502,6 +502,7 @@ k_row_solve(SolveArgs a, Op op) {
                     if (last) __threadfence();
                 }
                 if (!__shfl_sync(kFull, last, 0)) continue;
+                __syncwarp();   // lane 0 acquired; a shuffle orders no memory for the others
                 s = 0.0f;
                 c = 0.0f;
                 for (uint32_t q = lane; q < nseg; q += 32) {
