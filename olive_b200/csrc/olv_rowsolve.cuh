@@ -205,8 +205,11 @@ int build_solve_plan(const uint32_t *ptr, const uint32_t *idx, const uint32_t *e
 // Whether the stream may use every SM (it does not belong to a green context).
 bool stream_has_whole_gpu(cudaStream_t s);
 
-inline int solve_error(const SolveCtl &c, const char *what) {
+// After a solve of plan p on stream s has ended with control block c.  A run that gave up
+// may have left segments counted: the next one starts from zero again.
+inline int solve_error(const SolveCtl &c, const SolvePlan &p, cudaStream_t s, const char *what) {
     if (!c.err) return OLV_OK;
+    OLV_CUDA(cudaMemsetAsync(p.seg_done.p, 0, (size_t)p.nlong * 4, s));
     set_error("%s: a grid barrier ran out of time", what);
     return OLV_ERR_TIMEOUT;
 }

@@ -434,7 +434,7 @@ extern "C" int olv_pagerank(olv_graph *g, double alpha, int max_it, double tol, 
     if (!dev_out)
         OLV_CUDA(cudaMemcpyAsync(rank_out, rank, (size_t)g->V * 4, cudaMemcpyDeviceToHost, s));
     OLV_CUDA(cudaStreamSynchronize(s));
-    OLV_TRY(solve_error(hs, "olv_pagerank"));
+    OLV_TRY(solve_error(hs, p.sp, s, "olv_pagerank"));
     if (p.solve) {
         hc.iter = hs.iter;
         hc.residual = hs.residual;

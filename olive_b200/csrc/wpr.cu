@@ -376,8 +376,9 @@ extern "C" int olv_wpr_forward(olv_graph *g, const float *w, const float *p, dou
     OLV_CUDA(cudaMemcpyAsync(&hr, rctl, sizeof hr, cudaMemcpyDeviceToHost, s));
     if (r_out) OLV_CUDA(cudaMemcpyAsync(r_out, c->r.p, V * 4, cudaMemcpyDefault, s));
     OLV_CUDA(cudaStreamSynchronize(s));
-    OLV_TRY(solve_error(hc, "olv_wpr_forward"));
-    OLV_TRY(solve_error(hr, "olv_wpr_forward"));
+    const int solved = solve_error(hc, pl.tcsc, s, "olv_wpr_forward");
+    OLV_TRY(solve_error(hr, pl.tcsr, s, "olv_wpr_forward"));
+    OLV_TRY(solved);
     if (st) {
         float ms = 0;
         OLV_CUDA(cudaEventElapsedTime(&ms, g->ev0, g->ev1));
@@ -464,8 +465,8 @@ extern "C" int olv_wpr_backward(olv_wpr_ctx *c, const float *gvec, int max_it, d
     if (!dev_dw) OLV_CUDA(cudaMemcpyAsync(dw_out, dw, E * 4, cudaMemcpyDeviceToHost, s));
     if (dp_out && !dev_dp) OLV_CUDA(cudaMemcpyAsync(dp_out, dp, V * 4, cudaMemcpyDeviceToHost, s));
     OLV_CUDA(cudaStreamSynchronize(s));
-    OLV_TRY(solve_error(hc, "olv_wpr_backward"));
-    OLV_TRY(solve_error(ht, "olv_wpr_backward"));
+    OLV_TRY(solve_error(hc, pl.tcsr, s, "olv_wpr_backward"));
+    OLV_TRY(solve_error(ht, pl.tcsr, s, "olv_wpr_backward"));
     if (st) {
         float ms = 0;
         OLV_CUDA(cudaEventElapsedTime(&ms, g->ev0, g->ev1));
