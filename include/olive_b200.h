@@ -98,9 +98,12 @@ int olv_graph_destroy(olv_graph *g);
 int olv_graph_info(const olv_graph *g, uint32_t *V, uint64_t *E, int *weight_type);
 /* Copy the CSR back (any of the pointers may be NULL). */
 int olv_graph_copy_csr(const olv_graph *g, uint32_t *rowptr, uint32_t *col, void *weights);
-/* Replace the FP32 edge weights (CSR order) without rebuilding the graph.   */
+/* Replace the FP32 edge weights (CSR order) without rebuilding the graph.  The copy
+ * is stream-ordered: w must keep its values until the handle's stream has passed it
+ * (pageable host memory may be reused at once).                              */
 int olv_graph_set_weights_f32(olv_graph *g, const float *w);
-/* Bind the handle to a CUDA stream (a cudaStream_t; NULL = the handle's own). */
+/* Bind the handle to a CUDA stream (a cudaStream_t; NULL = the handle's own).  Work of
+ * the handle still under way on the last one comes before the new one's.     */
 int olv_set_stream(olv_graph *g, void *stream);
 /* Device memory that handles gave up is kept for the next buffers, at most 1/64
  * of the device's memory (no reference counterpart).  This call gives what is

@@ -298,6 +298,7 @@ class Graph:
 
     def set_weights_f32(self, w):
         w = np.ascontiguousarray(w, np.float32) if not hasattr(w, "data_ptr") else w.contiguous()
+        self._weights = w   # the copy is stream-ordered: not given up before a call has waited
         _check(lib().olv_graph_set_weights_f32(self._h, _ptr(w)), "olv_graph_set_weights_f32")
         self.weight_type = W_F32
 
@@ -372,6 +373,7 @@ class Graph:
                "olv_wpr_forward")
         if w is not None:
             self.weight_type = W_F32
+        self._weights = None
         self.last_stats = st
         return out
 

@@ -158,12 +158,17 @@ void put(const Block &b) {
 
 }  // namespace
 
-BufferScope::BufferScope(cudaStream_t s, bool keep) : before(t_stream), kept_before(t_keep) {
+BufferScope::BufferScope(cudaStream_t s)
+    : before(t_stream), kept_before(t_keep), errors_before(error_count()) {
     t_stream = s;
-    t_keep = keep;
+    t_keep = true;
 }
 
-BufferScope::~BufferScope() {
+void BufferScope::end() {
+    if (ended) return;
+    ended = true;
+    if (error_count() != errors_before && cudaStreamSynchronize(t_stream) != cudaSuccess)
+        cudaGetLastError();
     t_stream = before;
     t_keep = kept_before;
 }

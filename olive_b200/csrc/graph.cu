@@ -15,13 +15,17 @@
 namespace olv {
 
 static thread_local char g_err[512] = "";
+static thread_local unsigned g_errors = 0;
 
 void set_error(const char *fmt, ...) {
     va_list ap;
     va_start(ap, fmt);
     vsnprintf(g_err, sizeof g_err, fmt, ap);
     va_end(ap);
+    g_errors++;
 }
+
+unsigned error_count() { return g_errors; }
 
 int cuda_fail(cudaError_t e, const char *what, const char *file, int line) {
     set_error("%s failed: %s (%s:%d)", what, cudaGetErrorString(e), file, line);
@@ -329,6 +333,7 @@ int olv_graph_create(const uint32_t *rowptr, const uint32_t *col, const void *we
     if (r == OLV_OK) r = check_csr(g);
     if (r == OLV_OK) r = finish_graph(g);
     if (r != OLV_OK) {
+        scope.end();
         olv_graph_destroy(g);
         return r;
     }
@@ -423,6 +428,7 @@ int olv_graph_create_rmat(int scale, int edge_factor, uint64_t seed, int weight_
     }
     if (r == OLV_OK) r = finish_graph(g);
     if (r != OLV_OK) {
+        scope.end();
         olv_graph_destroy(g);
         return r;
     }
@@ -454,7 +460,8 @@ int olv_graph_destroy(olv_graph *g) {
     if (g->host_ctl) cudaFreeHost(g->host_ctl);
     if (g->ev0) cudaEventDestroy(g->ev0);
     if (g->ev1) cudaEventDestroy(g->ev1);
-    BufferScope none(nullptr, false);   // the stream goes
+    if (g->weights_in) cudaEventDestroy(g->weights_in);
+    scope.end();   // the stream goes
     if (g->own_stream) cudaStreamDestroy(g->own_stream);
     delete g;
     return OLV_OK;
@@ -483,9 +490,10 @@ int olv_graph_copy_csr(const olv_graph *g, uint32_t *rowptr, uint32_t *col, void
 
 int olv_graph_set_weights_f32(olv_graph *g, const float *w) {
     OLV_CHECK_ARG(g && (w || g->E == 0), "olv_graph_set_weights_f32: null pointer");
+    if (!g->weights_in)
+        OLV_CUDA(cudaEventCreateWithFlags(&g->weights_in, cudaEventDisableTiming));
     OLV_TRY(copy_in(g->w, w, g->E * 4, g->stream));
-    // the handle may be moved to another stream next, which would not wait for this
-    OLV_CUDA(cudaStreamSynchronize(g->stream));
+    OLV_CUDA(cudaEventRecord(g->weights_in, g->stream));   // olv_set_stream orders by it
     // no CSC copy: only SSSP reads one, and its weights are uint32
     g->weight_type = OLV_W_F32;
     return OLV_OK;
@@ -612,7 +620,10 @@ int olv_tune_get(const olv_graph *g, const char *key, double *value) {
 
 int olv_set_stream(olv_graph *g, void *stream) {
     OLV_CHECK_ARG(g, "olv_set_stream: null graph");
-    g->stream = stream ? (cudaStream_t)stream : g->own_stream;
+    const cudaStream_t s = stream ? (cudaStream_t)stream : g->own_stream;
+    // the one call that returns with work of the handle under way (others have waited)
+    if (g->weights_in && s != g->stream) OLV_CUDA(cudaStreamWaitEvent(s, g->weights_in, 0));
+    g->stream = s;
     return OLV_OK;
 }
 

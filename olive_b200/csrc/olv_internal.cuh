@@ -12,6 +12,7 @@ namespace olv {
 
 // ---------------------------------------------------------------- errors --
 void set_error(const char *fmt, ...);
+unsigned error_count();   // errors set on this thread so far
 int cuda_fail(cudaError_t e, const char *what, const char *file, int line);
 
 #define OLV_CUDA(call)                                                          \
@@ -51,17 +52,21 @@ struct DevBuf {
 };
 
 // While one stands, buffers that this thread gives up are kept for the next ones
-// once `s`, the only stream that uses them, is idle; otherwise they are freed.
+// once `s`, the only stream that uses them, is idle; otherwise they are freed.  A call
+// that fails on the way may leave work on `s`: the scope's end waits for it, so that it
+// is still the only one when the handle is moved to another stream next.
 class BufferScope {
 public:
-    explicit BufferScope(cudaStream_t s, bool keep = true);
-    ~BufferScope();
+    explicit BufferScope(cudaStream_t s);
+    ~BufferScope() { end(); }
+    void end();   // now, as before the stream is destroyed
     BufferScope(const BufferScope &) = delete;
     BufferScope &operator=(const BufferScope &) = delete;
 
 private:
     cudaStream_t before;
-    bool kept_before;
+    bool kept_before, ended = false;
+    unsigned errors_before;
 };
 
 // Where a caller's pointer lives.
@@ -157,6 +162,7 @@ struct olv_graph {
     olv::Tuning tune;
     olv::TravCtl *host_ctl = nullptr;   // pinned mirror of the control block
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t weights_in = nullptr;   // after the last copy of olv_graph_set_weights_f32
     uint32_t max_out_degree = 0;
     uint32_t max_in_degree = 0;
     int persist_blocks = 0;              // resident CTAs of kBlock threads (all SMs)
