@@ -101,7 +101,7 @@ __global__ void k_fill_i32(int32_t *__restrict__ a, uint32_t n, int32_t x) {
 // a 128 x 128 grid (about 200 levels): 3.94 -> 0.42 ms a call; the first and
 // last levels of a uniform digraph of 1,000,003 vertices: 380 -> 289 us, of
 // RMAT-24: 594 -> 554 us (there also two launches fewer per superstep).
-struct SmallShared {
+struct BfsSmallShared {
     SmallIndex ix;                                            // the level being expanded
     uint32_t v[kSmallCap], obeg[kSmallCap], odeg[kSmallCap];  // the next one
     uint32_t n;
@@ -145,7 +145,7 @@ __device__ __forceinline__ uint32_t bfs_small_edges(uint32_t base, uint32_t tota
                                                     int32_t *level, uint32_t *q,
                                                     const uint32_t *__restrict__ rowptr,
                                                     const uint32_t *__restrict__ col,
-                                                    SmallShared &sh) {
+                                                    BfsSmallShared &sh) {
     // each stage issues all its loads or atomics before any result is used
     uint32_t at[N], v[N], rb[N], re[N], pos[N], found = 0;
     int was[N];
@@ -190,7 +190,7 @@ __device__ __forceinline__ uint32_t bfs_small_edges(uint32_t base, uint32_t tota
 // large; leaves the frontier in the same queue.
 __device__ void bfs_small(TravCtl *c, uint32_t *q0, uint32_t *q1,
                           const uint32_t *__restrict__ rowptr, const uint32_t *__restrict__ col,
-                          SmallShared &sh) {
+                          BfsSmallShared &sh) {
     int32_t *level = static_cast<int32_t *>(c->vdata);
     uint32_t *q = c->cur ? q1 : q0;
     uint32_t n = c->qsize[c->cur];
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(kSmallThreads)
 k_bfs_init(TravCtl *c, int32_t *level, uint32_t *q0, uint32_t *q1, const uint32_t *rowptr,
            const uint32_t *col, uint32_t src, uint32_t V, unsigned long long E, int fill,
            float alpha, float beta, cudaGraphConditionalHandle h, int use_cond) {
-    __shared__ SmallShared sh;
+    __shared__ BfsSmallShared sh;
     if (fill) {
         for (uint32_t i = threadIdx.x; i < V; i += kSmallThreads) level[i] = kInf;
         __syncthreads();
@@ -626,7 +626,7 @@ k_bfs_pull_overflow(const uint32_t *__restrict__ colptr, const uint32_t *__restr
 __global__ void __launch_bounds__(kSmallThreads)
 k_bfs_end(TravCtl *c, cudaGraphConditionalHandle h, int use_cond, uint32_t V, uint32_t *q0,
           uint32_t *q1, const uint32_t *rowptr, const uint32_t *col, float alpha, float beta) {
-    __shared__ SmallShared sh;
+    __shared__ BfsSmallShared sh;
     if (threadIdx.x == 0) {
         if (!c->done) {
             c->edges_traversed += c->m_f;

@@ -876,7 +876,7 @@ struct SsspSmall {
     uint32_t bl_cap, max_steps;
 };
 
-struct SmallShared {
+struct SsspSmallShared {
     TravCtl c;
     uint32_t din[kSmallCap];                   // the superstep's input: distances
     SmallIndex ix;                             // its edges
@@ -902,7 +902,7 @@ __device__ __forceinline__ uint2 small_range(const SsspSmall &x, bool all, uint3
 // Entry pos of the near queue: in shared memory with its row range, or past
 // its capacity in the global queue.
 __device__ __forceinline__ void small_put(uint32_t pos, uint32_t v, uint2 r, uint32_t *q,
-                                          SmallShared &sh) {
+                                          SsspSmallShared &sh) {
     if (pos < kSmallCap) {
         sh.v[pos] = v;
         sh.obeg[pos] = r.x;
@@ -926,7 +926,7 @@ struct SmallStep {
 template <int N>
 __device__ __forceinline__ void small_edges(const SsspSmall &x, const SmallStep &a, uint32_t base,
                                             uint32_t total, uint32_t *dist, uint32_t &fmin,
-                                            SmallShared &sh) {
+                                            SsspSmallShared &sh) {
     // each stage issues all its loads or atomics before any result is used
     uint32_t at[N], du[N], old[N], nd[N], pos[N];
     uint2 e[N], r[N];
@@ -990,7 +990,7 @@ __device__ __forceinline__ void small_edges(const SsspSmall &x, const SmallStep 
 // until it is empty or does not fit.  Between two of them only the queue and
 // the counters move on, kept by every thread alike; the end step of the one
 // that empties the queue is left to the caller (returns true).
-__device__ bool small_relax(const SsspSmall &x, uint32_t n, uint32_t *dist, SmallShared &sh) {
+__device__ bool small_relax(const SsspSmall &x, uint32_t n, uint32_t *dist, SsspSmallShared &sh) {
     const uint32_t t = threadIdx.x;
     SmallStep a;
     a.all = sh.c.mode == kModeRelaxAll;
@@ -1070,7 +1070,7 @@ __device__ bool small_relax(const SsspSmall &x, uint32_t n, uint32_t *dist, Smal
 
 // One split of the far pile (as sssp_split): entries under the old threshold
 // are dropped, those under the new one are queued, the rest move on.
-__device__ void small_split(const SsspSmall &x, const uint32_t *dist, SmallShared &sh) {
+__device__ void small_split(const SsspSmall &x, const uint32_t *dist, SsspSmallShared &sh) {
     const uint32_t fc = sh.c.far_cur, n = sh.c.far_size[fc];
     const uint32_t *fin = fc ? x.far1 : x.far0;
     uint32_t *fout = fc ? x.far0 : x.far1;
@@ -1128,7 +1128,7 @@ __device__ void small_split(const SsspSmall &x, const uint32_t *dist, SmallShare
 
 // The near queue for the kernel chain: each vertex once, in the global queue,
 // with its near mark set (the chain's next superstep clears it).
-__device__ void small_leave(const SsspSmall &x, SmallShared &sh) {
+__device__ void small_leave(const SsspSmall &x, SsspSmallShared &sh) {
     const uint32_t n = sh.c.qsize[sh.c.cur];
     if (n == 0) return;
     const uint32_t *qin = sh.c.cur ? x.q1 : x.q0;
@@ -1159,7 +1159,7 @@ __device__ void small_leave(const SsspSmall &x, SmallShared &sh) {
 
 // Whole CTA: supersteps from the control block's state (its mode chosen) until
 // one does not fit or the run is over.  sh.c holds the control block.
-__device__ void sssp_small(const SsspSmall &x, cudaGraphConditionalHandle h, SmallShared &sh) {
+__device__ void sssp_small(const SsspSmall &x, cudaGraphConditionalHandle h, SsspSmallShared &sh) {
     uint32_t *dist = static_cast<uint32_t *>(sh.c.vdata);
     bool loaded = false;   // the near queue is in shared memory (the same in every thread)
     while (sssp_small_ok(sh.c)) {
@@ -1198,7 +1198,7 @@ struct SsspStart {
 
 __global__ void __launch_bounds__(kSmallThreads)
 k_sssp_init(TravCtl *c, SsspStart a, SsspSmall x, cudaGraphConditionalHandle h, int use_cond) {
-    __shared__ SmallShared sh;
+    __shared__ SsspSmallShared sh;
     if (threadIdx.x == 0) {
         const uint32_t src = a.newid ? a.newid[a.src] : a.src;
         TravCtl t = {};
@@ -1238,7 +1238,7 @@ k_sssp_init(TravCtl *c, SsspStart a, SsspSmall x, cudaGraphConditionalHandle h, 
 
 __global__ void __launch_bounds__(kSmallThreads)
 k_sssp_end(TravCtl *c, cudaGraphConditionalHandle h, int use_cond, SsspSmall x) {
-    __shared__ SmallShared sh;
+    __shared__ SsspSmallShared sh;
     if (threadIdx.x == 0) {
         sh.c = *c;
         sssp_end_step(&sh.c, h, 0, x.max_steps, x.bl_cap);
