@@ -152,7 +152,9 @@ int olv_graph_max_degree_vertex(const olv_graph *g, uint32_t *v, uint32_t *deg);
  *   "ms_alpha"    msBFS pull when active out-edges * ms_alpha > E   (20)
  *   "pr_tile_u"   PageRank / weighted PageRank: entries per lane per round
  *                 the row grouping aims at (1..32, a power of two); sets
- *                 the lanes per row of the tile plans, rebuilt on change;
+ *                 the lanes per row of the row plans, rebuilt on change (solves
+ *                 in one launch use at most 4 below 5120 edges per SM, and
+ *                 choose for themselves up to 8192 rows and 196,608 edges);
  *                 a weighted-PR backward needs its forward run after it (8)
  *   "use_graphs"  run supersteps inside CUDA graphs (1) or a host loop (0)
  *                 (solves that run in one launch, as weighted PageRank's, ignore it)

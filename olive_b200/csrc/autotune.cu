@@ -96,8 +96,11 @@ extern "C" int olv_autotune(olv_graph *g, const char *json_path, int reps) {
         plan.push_back({"sssp_piece", {256, 1024}, run_sssp, out.p});
         plan.push_back({"sssp_sub", {0, 8, 16}, run_sssp, out.p});
     }
-    // PageRank / weighted PageRank row grouping (entries per lane per round)
-    plan.push_back({"pr_tile_u", {4, 8, 16}, run_pagerank, out.p});
+    // PageRank / weighted PageRank row grouping (entries per lane per round), where the
+    // plan follows it
+    std::vector<double> lanes = {4, 8, 16};
+    if (!pr_tile_u_matters(g)) lanes = {(double)g->tune.pr_tile_u};
+    plan.push_back({"pr_tile_u", lanes, run_pagerank, out.p});
     // multi-source BFS push -> pull switch point
     std::vector<uint32_t> rp((size_t)g->V + 1);
     OLV_TRY(olv_graph_copy_csr(g, rp.data(), nullptr, nullptr));

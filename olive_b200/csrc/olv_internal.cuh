@@ -179,6 +179,8 @@ namespace olv {
 // Resident CTAs of kBlock threads for `kernel` on all SMs (a persistent grid).
 int resident_blocks(const olv_graph *g, const void *kernel, int *blocks);
 void release_pr_state(olv_graph *g);
+// Whether PageRank's plan of this graph follows the tunable pr_tile_u (pagerank.cu).
+bool pr_tile_u_matters(const olv_graph *g);
 void release_ppr_state(olv_graph *g);
 void release_ms_state(olv_graph *g);
 void release_wpr_state(olv_graph *g);

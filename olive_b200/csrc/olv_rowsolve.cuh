@@ -193,6 +193,12 @@ int permuted_offsets(const uint32_t *ptr, const uint32_t *perm, uint32_t n, cuda
 // Rows longer than bounds[i], i < nb <= 8, of rows sorted by length (sorted_ptr).
 int rows_longer(const uint32_t *sorted_ptr, uint32_t n, const uint32_t *bounds, int nb,
                 cudaStream_t s, uint32_t *counts);
+// Whether a solve plan of n rows and nnz entries takes the lanes_u it is given; smaller
+// ones choose their own (at most four entries per lane, or a cluster's).
+inline bool solve_lanes_free(uint64_t nnz, uint32_t n, int num_sms) {
+    return !(n <= kClusterRows && nnz <= kClusterEntries) &&
+           nnz >= (uint64_t)num_sms * kSolveMinBlocks * kBlock * 4;
+}
 // The whole plan.  lanes_u: entries per lane the grouping aims at (rows get the
 // fewest lanes G with G * lanes_u >= length; fewer entries per lane where that
 // leaves SMs idle); with_pos: keep each entry's position in the structure

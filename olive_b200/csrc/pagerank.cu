@@ -273,6 +273,10 @@ static bool one_launch(const olv_graph *g) {
     return rows_long_enough && (g->max_in_degree <= kRowLong || (few && g->V <= 3u << 17));
 }
 
+bool pr_tile_u_matters(const olv_graph *g) {
+    return !one_launch(g) || solve_lanes_free(g->E, g->V, g->num_sms);
+}
+
 static int build_pr_plan(olv_graph *g, PrPlan &p) {
     const uint32_t V = g->V;
     p.solve = one_launch(g);

@@ -346,7 +346,7 @@ int build_solve_plan(const uint32_t *ptr, const uint32_t *idx, const uint32_t *e
     if (p.cluster) {
         lanes_u = 4;
         while (lanes_u < 16 && (uint64_t)lanes_u * kClusterCTAs * kClusterThreads < nnz) lanes_u *= 2;
-    } else if (lanes_u > 4 && nnz < (uint64_t)num_sms * kSolveMinBlocks * kBlock * 4) {
+    } else if (lanes_u > 4 && !solve_lanes_free(nnz, n, num_sms)) {
         lanes_u = 4;
     }
     DevBuf sptr;
