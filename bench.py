@@ -465,23 +465,9 @@ def traversal_line(a, rank, world, local_rank, extra_keys=True):
     if traffic:
         roofline["traffic_over_algorithmic"] = round(traffic / alg_bytes, 3)
 
-    # launches of our kernels per step (kernel nodes executed by the graph).
-    # Supersteps of small frontiers run inside the kernel that begins the run or
-    # ends a superstep, so for sssp and bfs the count is a lower bound: the
-    # supersteps that pulled are certain to have run the whole chain.
-    # sssp: fill, init, 4 per superstep, the map back to the caller's ids
-    # (renumbered run), reached count; bfs: fill, init, 7 per level; msbfs:
-    # init, 5 per level, levels; pagerank: init, control, 3 per iteration, map
-    # back, or init, one solve kernel, map back
-    if a.workload == "sssp":
-        per_step = 2 + 4 * st.pull_steps + 1 + int(g.tune().get("sssp_relabel", 0))
-    elif a.workload == "bfs":
-        per_step = 2 + 7 * st.pull_steps
-    elif a.workload == "msbfs":
-        per_step = 2 + 5 * st.iterations
-    else:
-        per_step = 3 if E < 3 << 20 else 3 + 3 * st.iterations
-    launches = per_step * a.steps
+    # launches of our kernels per step: the library's own count of the last one (a
+    # superstep loop's kernels counted on the device; every step runs the same solve)
+    launches = g.last_launches() * a.steps
 
     # end to end through the public API: host (pinned) output buffer, D2H inside
     host_out = torch.empty(out.shape, dtype=out.dtype, pin_memory=True)
@@ -891,6 +877,7 @@ def ppr_line(a, rank, world, local_rank):
     barrier(world)
     ms = max_over_ranks(timed(stream, step, a.steps), world)
     clk = clocks.stop()
+    launches = g.last_launches()
     st = g.last_stats
     it = st.iterations
     units = E * it                                  # edge visits (each carries K values)
@@ -934,7 +921,7 @@ def ppr_line(a, rank, world, local_rank):
     config["workload"] = f"ppr32-rmat{a.scale}"
     line = common_line(a, world, "GE/s/iter", value, ms, "f32",
                        "synthetic (seeded RMAT, generated on the device)", config, roofline,
-                       None, e2e, a.steps * (3 * it + 3), clk, extra)
+                       None, e2e, a.steps * launches, clk, extra)
     g.close()
     return line
 

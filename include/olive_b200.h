@@ -105,6 +105,9 @@ int olv_graph_set_weights_f32(olv_graph *g, const float *w);
 /* Bind the handle to a CUDA stream (a cudaStream_t; NULL = the handle's own).  Work of
  * the handle still under way on the last one comes before the new one's.     */
 int olv_set_stream(olv_graph *g, void *stream);
+/* Kernels launched by the last solve on the handle (a superstep loop's by the device's
+ * own count), without those that build what a handle keeps.                  */
+int olv_last_launches(const olv_graph *g, uint64_t *kernels);
 /* Device memory that handles gave up is kept for the next buffers, at most 1/64
  * of the device's memory (no reference counterpart).  This call gives what is
  * kept in the calling thread's context back to the driver, for the other users

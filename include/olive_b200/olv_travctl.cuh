@@ -59,6 +59,7 @@ struct TravCtl {
     uint32_t ms_sparse_from;    // msBFS: first level applied sparsely (no store slot)
     uint32_t ms_cur_dense;      // msBFS: the frontier array is valid at every vertex
     unsigned long long ms_new_prev, ms_new_prev2;   // msBFS: vertices found one / two levels ago
+    uint32_t chains;            // BFS, SSSP: supersteps run by the kernel chain (not by one CTA)
     void *vdata;                // per-vertex result array of the run (level / dist)
     unsigned long long m_f;         // out-edges of the input frontier
     unsigned long long m_next;      // out-edges of vertices discovered this superstep

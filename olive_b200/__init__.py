@@ -86,6 +86,7 @@ _SIGS = [
     ("olv_graph_copy_csr", _I, [_VP, _VP, _VP, _VP]),
     ("olv_graph_set_weights_f32", _I, [_VP, _VP]),
     ("olv_set_stream", _I, [_VP, _VP]),
+    ("olv_last_launches", _I, [_VP, ctypes.POINTER(_U64)]),
     ("olv_release_memory", _I, [ctypes.POINTER(_U64)]),
     ("olv_graph_max_degree_vertex", _I, [_VP, ctypes.POINTER(_U32), ctypes.POINTER(_U32)]),
     ("olv_tune_set", _I, [_VP, ctypes.c_char_p, _D]),
@@ -267,6 +268,12 @@ class Graph:
         _check(lib().olv_graph_max_degree_vertex(self._h, ctypes.byref(v), ctypes.byref(d)),
                "olv_graph_max_degree_vertex")
         return v.value, d.value
+
+    def last_launches(self):
+        """Kernels the last solve launched (olv_last_launches)."""
+        n = _U64()
+        _check(lib().olv_last_launches(self._h, ctypes.byref(n)), "olv_last_launches")
+        return n.value
 
     def tune(self, **kw):
         """Set engine tunables (see olv_tune_set); returns the current values."""

@@ -902,6 +902,7 @@ extern "C" int olv_batch_run(olv_graph *g, const uint32_t *inst_offsets, int cou
     if (ppr_iters_out)
         OLV_CUDA(cudaMemcpyAsync(ppr_iters_out, bs.iters.p, count * 4, cudaMemcpyDefault, s));
     OLV_CUDA(cudaStreamSynchronize(s));
+    g->launches = 1;
     if (hst[2]) {
         set_error("olv_batch_run: the graph is not block-diagonal under inst_offsets "
                   "(edges cross instances; code %llu)", hst[2]);

@@ -629,6 +629,7 @@ k_bfs_end(TravCtl *c, cudaGraphConditionalHandle h, int use_cond, uint32_t V, ui
     __shared__ BfsSmallShared sh;
     if (threadIdx.x == 0) {
         if (!c->done) {
+            c->chains++;
             c->edges_traversed += c->m_f;
             c->reached += c->qsize[c->cur];
             if (c->mode) c->pull_steps++;
@@ -825,7 +826,9 @@ static AdvanceArgs bfs_adv_args(olv_graph *g) {
     return a;
 }
 
-// One superstep's kernel chain, either launched on a stream or added to a graph.
+// One superstep's kernel chain (kBfsChain kernels), either launched on a stream or added
+// to a graph.
+constexpr int kBfsChain = 7;
 template <class Sink>
 static int bfs_superstep(olv_graph *g, Sink &&sink, cudaGraphConditionalHandle h, int use_cond) {
     TravCtl *ctl = g->ws.ctl.as<TravCtl>();
@@ -914,6 +917,8 @@ int run_bfs_device(olv_graph *g, uint32_t src, int32_t *level_dev) {
     if (!fill_here) k_fill_i32<<<g->num_sms * 8, kBlock, 0, s>>>(level_dev, g->V, kInf);
     OLV_CUDA(cudaGetLastError());
     BfsInitArgs init(g, src, level_dev, fill_here);
+    g->launches = 1 + !fill_here;
+    g->chain_kernels = kBfsChain;
     if (g->tune.use_graphs) {
         if (bfs_graph(g, init) == OLV_OK) return g->bfs_graph->launch(s);
         g->tune.use_graphs = 0;   // conditional graphs unavailable: host loop below
@@ -925,8 +930,10 @@ int run_bfs_device(olv_graph *g, uint32_t src, int32_t *level_dev) {
         OLV_CUDA(cudaLaunchKernel(f, gr, bl, args, 0, s));
         return OLV_OK;
     };
+    g->chain_kernels = 0;   // every launch is counted here
     for (;;) {
         for (int i = 0; i < g->tune.levels_per_sync; i++) OLV_TRY(bfs_superstep(g, launch, 0, 0));
+        g->launches += (uint64_t)kBfsChain * g->tune.levels_per_sync;
         OLV_CUDA(cudaMemcpyAsync(g->host_ctl, ctl, sizeof(TravCtl), cudaMemcpyDeviceToHost, s));
         OLV_CUDA(cudaStreamSynchronize(s));
         if (g->host_ctl->done) break;
@@ -956,6 +963,7 @@ extern "C" int olv_bfs(olv_graph *g, uint32_t src, int32_t *level_out, olv_stats
         OLV_CUDA(cudaMemcpyAsync(level_out, level, (size_t)g->V * 4, cudaMemcpyDeviceToHost, s));
     OLV_CUDA(cudaStreamSynchronize(s));
     const TravCtl &h = *g->host_ctl;
+    g->launches += (uint64_t)g->chain_kernels * h.chains;
     if (h.err) {
         set_error("olv_bfs: device-side check failed (code %u)", h.err);
         return OLV_ERR_STATE;

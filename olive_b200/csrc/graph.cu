@@ -627,6 +627,12 @@ int olv_set_stream(olv_graph *g, void *stream) {
     return OLV_OK;
 }
 
+int olv_last_launches(const olv_graph *g, uint64_t *kernels) {
+    OLV_CHECK_ARG(g && kernels, "olv_last_launches: null pointer");
+    *kernels = g->launches;
+    return OLV_OK;
+}
+
 int olv_graph_max_degree_vertex(const olv_graph *g, uint32_t *v, uint32_t *deg) {
     OLV_CHECK_ARG(g && v, "olv_graph_max_degree_vertex: null pointer");
     DevBuf best;

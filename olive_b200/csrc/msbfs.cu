@@ -628,6 +628,7 @@ k_ms_levels4(uint32_t V, int n, unsigned long long srcmask, TravCtl *c,
 }
 
 // ------------------------------------------------------------------ host --
+constexpr int kMsChain = 5;   // kernels of a superstep
 template <class Sink>
 static int ms_superstep(olv_graph *g, MsState &ms, Sink &&sink, cudaGraphConditionalHandle h,
                         int use_cond, unsigned long long srcmask) {
@@ -774,6 +775,8 @@ extern "C" int olv_msbfs(olv_graph *g, const uint32_t *srcs, int n, int32_t *lev
                                g->tune.ms_alpha);
     OLV_CUDA(cudaGetLastError());
     bool launched = false;
+    g->launches = 2;
+    g->chain_kernels = kMsChain;
     if (g->tune.use_graphs) {
         if (!ms.graph.ready || ms.graph_n != (uint32_t)n) {
             int r = ms.graph.begin();
@@ -795,7 +798,9 @@ extern "C" int olv_msbfs(olv_graph *g, const uint32_t *srcs, int n, int32_t *lev
             OLV_CUDA(cudaLaunchKernel(f, gr, bl, args, 0, s));
             return OLV_OK;
         };
+        g->chain_kernels = 0;   // every launch is counted here
         for (;;) {
+            g->launches += (uint64_t)kMsChain * g->tune.levels_per_sync;
             for (int i = 0; i < g->tune.levels_per_sync; i++)
                 OLV_TRY(ms_superstep(g, ms, launch, 0, 0, srcmask));
             OLV_CUDA(cudaMemcpyAsync(g->host_ctl, ctl, sizeof(TravCtl), cudaMemcpyDeviceToHost, s));
@@ -819,6 +824,7 @@ extern "C" int olv_msbfs(olv_graph *g, const uint32_t *srcs, int n, int32_t *lev
     if (!dev_out) OLV_CUDA(cudaMemcpyAsync(levels_out, levels, out_bytes, cudaMemcpyDeviceToHost, s));
     OLV_CUDA(cudaStreamSynchronize(s));
     const TravCtl &h = *g->host_ctl;
+    g->launches += (uint64_t)g->chain_kernels * h.steps;
     if (h.err) {
         set_error("olv_msbfs: device-side check failed (code %u)", h.err);
         return OLV_ERR_STATE;

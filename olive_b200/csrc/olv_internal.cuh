@@ -162,6 +162,8 @@ struct olv_graph {
     olv::Tuning tune;
     olv::TravCtl *host_ctl = nullptr;   // pinned mirror of the control block
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    uint64_t launches = 0;              // kernels of the last solve (olv_last_launches)
+    int chain_kernels = 0;              // of a superstep's chain, where the device counts them
     cudaEvent_t weights_in = nullptr;   // after the last copy of olv_graph_set_weights_f32
     uint32_t max_out_degree = 0;
     uint32_t max_in_degree = 0;

@@ -373,6 +373,7 @@ extern "C" int olv_pagerank(olv_graph *g, double alpha, int max_it, double tol, 
 
     const uint32_t leak = dangling_mode == OLV_DANGLING_LEAK ? 1u : 0u;
     SolveCtl *sctl = p.sp.ctl.as<SolveCtl>();
+    bool launched = false;   // the passes as one graph
     OLV_CUDA(cudaEventRecord(g->ev0, s));
     if (p.solve)
         OLV_CUDA(cudaMemsetAsync(sctl, 0, sizeof(SolveCtl), s));
@@ -400,7 +401,6 @@ extern "C" int olv_pagerank(olv_graph *g, double alpha, int max_it, double tol, 
         k_pr_ctl_init<<<1, 1, 0, s>>>(p.ctl.as<PrCtl>(), p.dang.as<unsigned long long>(), g->V, ad,
                                       (uint32_t)max_it, tol, leak);
         OLV_CUDA(cudaGetLastError());
-        bool launched = false;
         if (g->tune.use_graphs && max_it > 0) {
             if (ps->graph.ready && ps->graph_alpha != ad) ps->graph.destroy();
             if (!ps->graph.ready) {
@@ -439,9 +439,12 @@ extern "C" int olv_pagerank(olv_graph *g, double alpha, int max_it, double tol, 
         OLV_CUDA(cudaMemcpyAsync(rank_out, rank, (size_t)g->V * 4, cudaMemcpyDeviceToHost, s));
     OLV_CUDA(cudaStreamSynchronize(s));
     OLV_TRY(solve_error(hs, p.sp, s, "olv_pagerank"));
+    g->launches = 3;   // init, one solve, map back
     if (p.solve) {
         hc.iter = hs.iter;
         hc.residual = hs.residual;
+    } else {   // init, control, the passes, map back
+        g->launches += (p.tp.nsegs ? 3ull : 2ull) * (launched ? hc.iter : (uint32_t)max_it);
     }
     if (st) {
         float ms = 0;

@@ -650,6 +650,8 @@ extern "C" int olv_ppr_batch(olv_graph *g, const uint32_t *seeds, int K, double 
     if (!dev_out)
         OLV_CUDA(cudaMemcpyAsync(out, dst, (size_t)g->V * K * 4, cudaMemcpyDeviceToHost, s));
     OLV_CUDA(cudaStreamSynchronize(s));
+    // seeds, start, the iterations, map back
+    g->launches = 3 + (p.nsegs ? 3ull : 2ull) * (launched ? hc.iter : (uint32_t)max_it);
     if (st) {
         float ms = 0;
         OLV_CUDA(cudaEventElapsedTime(&ms, g->ev0, g->ev1));

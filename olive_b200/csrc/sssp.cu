@@ -203,6 +203,7 @@ struct SsspOp {
     uint32_t end_max_steps, end_bl_cap;
     __device__ __forceinline__ bool epilogue_on() const { return end_fused != 0; }
     __device__ __forceinline__ void epilogue(TravCtl *c) const {
+        c->chains += !c->done;
         sssp_end_step(c, end_h, end_use_cond, end_max_steps, end_bl_cap);
     }
 
@@ -1241,6 +1242,7 @@ k_sssp_end(TravCtl *c, cudaGraphConditionalHandle h, int use_cond, SsspSmall x) 
     __shared__ SsspSmallShared sh;
     if (threadIdx.x == 0) {
         sh.c = *c;
+        sh.c.chains += !sh.c.done;
         sssp_end_step(&sh.c, h, 0, x.max_steps, x.bl_cap);
     }
     __syncthreads();
@@ -1696,6 +1698,9 @@ int run_sssp_device(olv_graph *g, uint32_t src, uint32_t *dist_dev, unsigned lon
                                ? std::max<uint32_t>(1u, g->V / 16) : 0u,
                            R.newid, dist, red};
     init.small = sssp_small_args(g);
+    const int chain = g->tune.sssp_fuse_end ? 3 : 4;   // sssp_superstep's kernels
+    g->launches = 2 + (R.dist ? 1 : 0);
+    g->chain_kernels = chain;
     auto finish = [&]() -> int {
         if (R.dist) {
             k_sssp_unrelabel<<<g->num_sms * 8, kBlock, 0, s>>>(R.dist, R.newid, g->V, dist_dev,
@@ -1719,8 +1724,10 @@ int run_sssp_device(olv_graph *g, uint32_t src, uint32_t *dist_dev, unsigned lon
         OLV_CUDA(cudaLaunchKernel(f, gr, bl, args, 0, s));
         return OLV_OK;
     };
+    g->chain_kernels = 0;   // every launch is counted here
     for (;;) {
         for (int i = 0; i < g->tune.levels_per_sync; i++) OLV_TRY(sssp_superstep(g, launch, 0, 0));
+        g->launches += (uint64_t)chain * g->tune.levels_per_sync;
         OLV_CUDA(cudaMemcpyAsync(g->host_ctl, ctl, sizeof(TravCtl), cudaMemcpyDeviceToHost, s));
         OLV_CUDA(cudaStreamSynchronize(s));
         if (g->host_ctl->done) break;
@@ -1754,15 +1761,18 @@ extern "C" int olv_sssp(olv_graph *g, uint32_t src, uint32_t *dist_out, olv_stat
     OLV_CUDA(cudaMemcpyAsync(g->host_ctl, g->ws.ctl.p, sizeof(TravCtl), cudaMemcpyDeviceToHost, s));
     unsigned long long red[2] = {0, 0};
     if (st) {
-        if (!red_done)
+        if (!red_done) {
             k_reached_edges<<<g->num_sms * 4, kBlock, 0, s>>>(g->rowptr.as<uint32_t>(), dist, g->V,
                                                              red_dev);
+            g->launches++;
+        }
         OLV_CUDA(cudaMemcpyAsync(red, red_dev, 16, cudaMemcpyDeviceToHost, s));
     }
     if (!dev_out)
         OLV_CUDA(cudaMemcpyAsync(dist_out, dist, (size_t)g->V * 4, cudaMemcpyDeviceToHost, s));
     OLV_CUDA(cudaStreamSynchronize(s));
     const TravCtl &h = *g->host_ctl;
+    g->launches += (uint64_t)g->chain_kernels * h.chains;
     if (h.err) {
         set_error("olv_sssp: device-side check failed (code %u)", h.err);
         return OLV_ERR_STATE;

@@ -379,6 +379,7 @@ extern "C" int olv_wpr_forward(olv_graph *g, const float *w, const float *p, dou
     const int solved = solve_error(hc, pl.tcsc, s, "olv_wpr_forward");
     OLV_TRY(solve_error(hr, pl.tcsr, s, "olv_wpr_forward"));
     OLV_TRY(solved);
+    g->launches = 6;   // two weight copies, their sums, init, one solve, map back
     if (st) {
         float ms = 0;
         OLV_CUDA(cudaEventElapsedTime(&ms, g->ev0, g->ev1));
@@ -467,6 +468,7 @@ extern "C" int olv_wpr_backward(olv_wpr_ctx *c, const float *gvec, int max_it, d
     OLV_CUDA(cudaStreamSynchronize(s));
     OLV_TRY(solve_error(hc, pl.tcsr, s, "olv_wpr_backward"));
     OLV_TRY(solve_error(ht, pl.tcsr, s, "olv_wpr_backward"));
+    g->launches = 3 + (E ? 1 : 0);   // init, one solve, the last sums, the edges' gradient
     if (st) {
         float ms = 0;
         OLV_CUDA(cudaEventElapsedTime(&ms, g->ev0, g->ev1));
