@@ -71,8 +71,8 @@ struct PrTileOp {
     const float *cin;
     float *cout;
     float a_hi, a_lo;   // alpha as an unevaluated FP32 pair: the update carries FP64-level
-                        // alpha (parameters: read from the control block they cost
-                        // 10-30 us of 4370 on RMAT-22, 20 iterations)
+                        // alpha (parameters: read from the control block they took two
+                        // registers more and were no faster)
     float base;
 
     __device__ __forceinline__ void begin() {

@@ -861,8 +861,8 @@ __device__ void sssp_end_step(TravCtl *c, cudaGraphConditionalHandle h, int use_
 // handed back, so a run can change over at any superstep.
 // What bounds it: dependent L2 round trips of one SM (about 4 us a superstep of
 // 1300 edges).  Measured: 301 x 517 grid, weights U[1,255], 815 supersteps
-// 13.9 -> 3.3 ms; RMAT-24 1.69 -> 1.67 ms (its last supersteps; also the
-// distances and marks cleared by one launch).
+// 13.9 -> 3.3 ms; RMAT-24, of whose supersteps only the last are small, 1.68 ms
+// before and after.
 constexpr uint32_t kSmallFar = 16384;
 constexpr uint32_t kSmallHash = 1024;
 
@@ -1435,8 +1435,8 @@ __global__ void k_sssp_unrelabel(const uint32_t *__restrict__ dnew,
     }
 }
 
-// Renumber the vertices by in-degree, highest first (a stable counting sort
-// on the host, once per graph), and build the CSR and CSC with weights in
+// Renumber the vertices by in-degree, highest first (a stable radix sort on
+// the device, once per graph), and build the CSR and CSC with weights in
 // the new ids.  The relax supersteps gather the distances of edge targets;
 // on a scale-free graph most gathers hit the high in-degree vertices, whose
 // distances then share cache lines instead of one 32-byte sector each.

@@ -7,7 +7,7 @@
 //   dL/dw_uv = alpha r_u (lambda_v - t_u) / W_u,   t_u = sum_x P_ux lambda_x
 //   dL/dp    = (1-alpha) lambda                     for L = sum_v g_v r_v.
 // Both solves are Jacobi sweeps with deterministic compensated FP32 row sums
-// and FP64 residual norms, run as CUDA graphs; the gradient is implicit at the
+// and FP64 residual norms, each solve one launch; the gradient is implicit at the
 // fixed point, so memory is O(V + E) with no tape.
 //
 // The row sums run on relabelled, row-sorted copies of the CSC (forward) and the
