@@ -37,7 +37,8 @@
 // An Op supplies:
 //   static constexpr bool kGather     entries gather a value of their neighbour
 //   static constexpr bool kWeighted   entries carry a weight
-//   static constexpr bool kStore      a row yields the value to gather next time
+//   static constexpr bool kStore      a row yields the value to gather next time; without,
+//                                     the solve is one pass (max_it 1) and has no sums
 //   double first_aux()                the aux sum before the first iteration
 //   void begin(uint32_t it, double aux)   iteration it (from 0) starts; aux: the
 //                                     last iteration's aux sum
@@ -296,7 +297,7 @@ k_row_solve(SolveArgs a, Op op) {
     const uint32_t ntiles = a.cls.tile0[kRowClasses], nfull = a.cls.tile0[kRowClasses - 1];
     const uint32_t nlong = a.cls.row0[1];
     uint32_t rank = blockIdx.x;
-    if constexpr (!kCluster) {
+    if constexpr (!kCluster && Op::kStore) {
         if (threadIdx.x == 0) {
             uint32_t r, n = 0;
             s_team = join_team(a.ctl, gridDim.x, r, n) ? n : 0;
@@ -391,7 +392,7 @@ k_row_solve(SolveArgs a, Op op) {
             if constexpr (!kCluster) {
                 u = s_first[wid].x;
                 ue = s_first[wid].y;
-                if (share >= s_team && gw < nfull) {   // not this CTA's first share
+                if (Op::kStore && share >= s_team && gw < nfull) {   // not this CTA's first share
                     u = __ldg(&a.units[gw]);
                     ue = __ldg(&a.units[gw + 1]);
                 }
@@ -536,6 +537,7 @@ k_row_solve(SolveArgs a, Op op) {
                 const uint32_t r = a.cls.row0[kRowClasses - 1] + (t - nfull) * 32 + lane;
                 if (r < a.nrows) end_row(r, 0.0f, 0.0f, op.row(r), res, aux);
             }
+            if constexpr (!Op::kStore) return;   // one pass: no barrier, no sums
             cta_sum(res, aux);
             if constexpr (kCluster) break;
             if (threadIdx.x == 0) {
