@@ -621,8 +621,14 @@ int olv_tune_get(const olv_graph *g, const char *key, double *value) {
 int olv_set_stream(olv_graph *g, void *stream) {
     OLV_CHECK_ARG(g, "olv_set_stream: null graph");
     const cudaStream_t s = stream ? (cudaStream_t)stream : g->own_stream;
-    // the one call that returns with work of the handle under way (others have waited)
-    if (g->weights_in && s != g->stream) OLV_CUDA(cudaStreamWaitEvent(s, g->weights_in, 0));
+    // the one call that returns with work of the handle under way (others have waited); a
+    // stream that is being captured cannot wait for what lies outside the capture
+    if (g->weights_in && s != g->stream) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        OLV_CUDA(cudaStreamIsCapturing(s, &capture));
+        if (capture == cudaStreamCaptureStatusNone)
+            OLV_CUDA(cudaStreamWaitEvent(s, g->weights_in, 0));
+    }
     g->stream = s;
     return OLV_OK;
 }

@@ -47,6 +47,25 @@ def test_weights_are_stream_ordered(torch):
     assert np.max(np.abs(r - ref)) < 1e-5 * np.max(ref)
 
 
+def test_moved_to_a_stream_under_capture(torch):
+    """Binding a handle neither ends nor joins the stream's capture."""
+    import olive_b200 as ob
+    rp, cl = oracle.rmat_csr(10, 8, 1)
+    x = torch.zeros(8, device="cuda")
+    with ob.Graph.from_csr(rp, cl) as g:
+        g.set_weights_f32(np.ones(len(cl), np.float32))
+        graph, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph, stream=s):
+            g.set_stream(s)
+            x += 1
+        g.set_stream(None)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert float(x[0]) == 1.0
+        assert np.array_equal(g.bfs(1), oracle.bfs(rp, cl, 1)[0])
+
+
 def test_closed_behind_a_busy_stream(torch):
     """The buffers of a handle that is moved away from a busy stream and closed are not
     handed out while the copy there is still to come."""
